@@ -17,7 +17,7 @@
 //           Phi(s)[P+] = D_W^dag Qp(s) + 2 R(s) - Qp(s),  Qp = R(s) + R(s+1) (wall z' R(1))
 // so the whole operator is again one pass over memory.
 //
-// The per-site arithmetic lives in shamir_site / wilson_site; the single-
+// The per-site arithmetic lives in shamir_site / wilson_exchange; the single-
 // lattice kernels and the batched kernel (many right-hand sides or many
 // lattices of different shapes in one persistent launch) share it.
 #include <cuda.h>
@@ -58,11 +58,11 @@ __device__ __forceinline__ void block_partial(double v, double* out) {
   __syncthreads();
 }
 
-// ---------------------------------------------------------------- overlap
-// The Zolotarev domain-wall operator of measure_OWilson.F90 (odslash :14-89,
-// odslashd :91-167): the Wilson-kernel operator with slice s's 3D Wilson term
-// D_W = DWilson(-am3) scaled by its coefficient c[s] (prepZolo, :169-188) and
-// the imass 3 walls of the opposite sign.  By linearity
+// ---------------------------------------------------------------- Wilson, overlap
+// The Wilson operator and the Zolotarev domain-wall operator of measure_OWilson.F90
+// (odslash :14-89, odslashd :91-167), which is the Wilson one with slice s's 3D Wilson
+// term D_W = DWilson(-am3) scaled by its coefficient c[s] (prepZolo, :169-188) and the
+// imass 3 walls of the opposite sign.  By linearity
 //   M:      Phi(s) = c[s] D_W Q(s) + 2 R(s) - Q(s),
 //           Q(s) = R(s) + P- R(s+1) + P+ R(s-1)   (walls: m1 P+ R(Ls) into s = 1,
 //           m2 P- R(1) into s = Ls; m1 = -am | +i am, m2 = -am | -i am)
@@ -70,99 +70,40 @@ __device__ __forceinline__ void block_partial(double v, double* out) {
 //           (s = Ls: c[Ls] R(Ls) + z2 c[1] R(1), non-D part R(Ls) - z2 R(1), z2 = -am | -i am)
 //           Phi(s)[P-] = D_W^dag(c[s] R(s) + c[s-1] R(s-1)) + R(s) - R(s-1)
 //           (s = 1: c[1] R(1) + z1 c[Ls] R(Ls), non-D part R(1) - z1 R(Ls), z1 = -am | +i am)
-// (1-based slices as in the reference).  One thread per 5D site, FP64.
-template <bool DAG>
-__device__ __forceinline__ void overlap_site(const double2* __restrict__ in, const double2* __restrict__ u,
-                                             const Geom& g, int s, int site, float am, int imass, float am3,
-                                             const double* __restrict__ zc, double2* res) {
-  using C = double2;
-  using R = double;
-  int x, y, t;
-  site_coords(g, site, x, y, t);
-  const Nbr nb = neighbours(g, site, x, y, t);
-  SpinorView<double2> Rv{in, g};
-  const int Ls = g.ls;
-  const R a = (R)am;
-  const R dgw = (R)(3.0f + (-am3));  // DWilson(..., -am3) diagonal: dirac.F90:191, :505
-  const R cs = __ldg(zc + s);
-  if (!DAG) {
-    const C m1 = imass == 1 ? mk(-a, R(0)) : mk(R(0), a);   // measure_OWilson.F90:66-71
-    const C m2 = imass == 1 ? mk(-a, R(0)) : mk(R(0), -a);  // :78-83
-    C q[4];
-    wilson_q<double2>(Rv, s, site, Ls, m1, m2, q);
-#pragma unroll
-    for (int d = 0; d < 4; d++) res[d] = (cs * dgw - R(1)) * q[d] + R(2) * Rv(s, site, d);
-#pragma unroll
-    for (int mu = 0; mu < 3; mu++) {
-      const C U = cs * __ldg(u + (size_t)mu * g.v3 + site);
-      const C Ub = cs * cconj(__ldg(u + (size_t)mu * g.v3 + nb.b[mu]));
-      wilson_q<double2>(Rv, s, nb.f[mu], Ls, m1, m2, q);
-      hop_projected<C, R>(mu, true, U, q, res);
-      wilson_q<double2>(Rv, s, nb.b[mu], Ls, m1, m2, q);
-      hop_projected<C, R>(mu, false, Ub, q, res);
-    }
-  } else {
-    const C z1 = imass == 1 ? mk(-a, R(0)) : mk(R(0), a);   // upper right, measure_OWilson.F90:139-144
-    const C z2 = imass == 1 ? mk(-a, R(0)) : mk(R(0), -a);  // lower left, :152-157
-    // output spins 0,1 from slice s+1 (wall: slice 0 with z2), spins 2,3 from s-1 (wall: Ls-1, z1);
-    // one pass over the neighbours loads R(s) and both partner slices once
-    const bool in0 = s < Ls - 1, in1 = s > 0;
-    const int sp0 = in0 ? s + 1 : 0, sp1 = in1 ? s - 1 : Ls - 1;
-    const R cn0 = __ldg(zc + sp0), cn1 = __ldg(zc + sp1);
-    const C zb0 = cn0 * z2, zb1 = cn1 * z1;
-    auto qpair = [&](int st, C* q0, C* q1) {
-#pragma unroll
-      for (int d = 0; d < 4; d++) {
-        const C r = Rv(s, st, d), a0 = Rv(sp0, st, d), a1 = Rv(sp1, st, d);
-        q0[d] = in0 ? cs * r + cn0 * a0 : cs * r + cmul(zb0, a0);
-        q1[d] = in1 ? cs * r + cn1 * a1 : cs * r + cmul(zb1, a1);
-      }
-    };
-    {
-      C q0[4], q1[4];
-      qpair(site, q0, q1);
-#pragma unroll
-      for (int d = 0; d < 4; d++) {
-        const bool lo = d < 2;
-        const C a2 = Rv(lo ? sp0 : sp1, site, d);
-        const C xo = (lo ? in0 : in1) ? a2 : cmul(lo ? z2 : z1, a2);
-        res[d] = dgw * (lo ? q0[d] : q1[d]) + Rv(s, site, d) - xo;
-      }
-    }
-#pragma unroll
-    for (int mu = 0; mu < 3; mu++) {
-      const C U = __ldg(u + (size_t)mu * g.v3 + site);
-      const C Ub = cconj(__ldg(u + (size_t)mu * g.v3 + nb.b[mu]));
-#pragma unroll
-      for (int dir = 0; dir < 2; dir++) {
-        C q0[4], q1[4];
-        qpair(dir == 0 ? nb.f[mu] : nb.b[mu], q0, q1);
-        const C W = dir == 0 ? U : Ub;
-#pragma unroll
-        for (int d = 0; d < 4; d++) {
-          const C* q = d < 2 ? q0 : q1;
-          const GammaEntry ge = gamma_entry(mu, d);
-          const C gq = gp(ge, q[ge.gin]);
-          res[d] = res[d] - R(0.5) * cmul(W, dir == 0 ? q[d] + gq : q[d] - gq);
-        }
-      }
-    }
-  }
-}
-
-// odslash / odslashd on one lattice: blockDim = (Ls, sites per block) as the Wilson kernel's
-template <bool DAG, int MINB>
-__global__ void __launch_bounds__(256, MINB)
-    k_odslash(double2* __restrict__ out, const double2* __restrict__ in, const double2* __restrict__ u, Geom g,
-              float am, int imass, float am3, const double* __restrict__ zc, const int* skip) {
+// (1-based slices as in the reference; Wilson: c = 1).  One thread per 5D site applies the
+// hops to its own slice, the slices combine through shared memory (wilson_exchange), so a
+// site costs 28 spinor loads, as the Shamir kernel, instead of the 56 to 84 that building
+// Q at every neighbour takes.  The epilogues (EPI) are k_dslash's.  MINB as there.
+// The Q-first kernel was bound by the L1 data path (67-80 %) and issued 770-1360
+// instructions per warp.  Measured against it (us per launch, M / M^dagger): overlap at
+// 48^2x48, Ls 16 74 / 60 instead of 110 / 147 (226 MB: 3.1 / 3.8 TB/s); Wilson at 24^2x24,
+// Ls 48, even-odd 30 / 26 instead of 44 / 48.  128-thread blocks, as the Shamir kernel's:
+// the exchange barrier then holds up four warps, not eight.
+template <class S, bool OV, bool DAG, int EPI, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
+    k_wilson(S* __restrict__ out, const S* __restrict__ in, const typename Sto<S>::C* __restrict__ u, Geom g, float am,
+             int imass, float am3, const double* __restrict__ zc, const int* skip, const S* __restrict__ aux,
+             const double* __restrict__ coef, double* __restrict__ partials, int rev) {
+  pdl_wait();
+  pdl_trigger();
   if (skip && *skip) return;
+  using C = typename Sto<S>::C;
+  using R = typename Sto<S>::R;
+  extern __shared__ __align__(16) unsigned char wsm[];
+  const R om = (EPI == 1 || EPI == 3) ? (R)(*coef) : R(0);
+  const int bid = rev ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
   const int s = threadIdx.x;
-  const int site = blockIdx.x * blockDim.y + threadIdx.y;
-  if (site >= g.v3) return;
-  double2 acc[4];
-  overlap_site<DAG>(in, u, g, s, site, am, imass, am3, zc, acc);
+  const int site = bid * (int)blockDim.y + threadIdx.y;
+  const bool live = site < g.v3;
+  C acc[4];
+  wilson_exchange<S, OV, DAG, NT>(in, u, g, s, site, live, s + (int)(blockDim.x * threadIdx.y), am, imass, am3, zc,
+                                  reinterpret_cast<C*>(wsm), acc);
+  double racc = 0.0;
+  if (live) {
 #pragma unroll
-  for (int d = 0; d < 4; d++) Sto<double2>::st(out, sidx32(g, s, site, d), acc[d]);
+    for (int d = 0; d < 4; d++) epi_element<S, EPI, false>(out, aux, om, sidx32(g, s, site, d), acc[d], racc);
+  }
+  if (EPI != 0) block_partial_sum<NT>(racc, partials, bid);
 }
 
 // ---------------------------------------------------------------- kernels
@@ -178,7 +119,7 @@ __global__ void __launch_bounds__(256, MINB)
 // aux + (*coef) * (M in), with M in never stored, and a partial of |out|^2;
 // 3 out = M in + (*coef) * aux with a partial of |out|^2 (the batched
 // multishift keeps h = M p by this recurrence instead of storing p).
-template <class S, int KER, bool DAG, int EPI, int NT, bool SHFL, int MINB>
+template <class S, bool DAG, int EPI, int NT, bool SHFL, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     k_dslash(S* __restrict__ out, const S* __restrict__ in, const typename Sto<S>::C* __restrict__ u, Geom g, float am,
              int imass, float am3, const int* skip, const S* __restrict__ aux, const double* __restrict__ coef,
@@ -191,7 +132,7 @@ __global__ void __launch_bounds__(NT, MINB)
   // rev: blocks walk the sites from the top, so that the first blocks find the
   // end of a field the previous kernel has just written still in L2
   const int bid = rev ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
-  dslash_block<S, KER, DAG, EPI, NT, SHFL>(out, in, u, g, am, imass, am3, aux, om, bid, partials);
+  dslash_block<S, DAG, EPI, NT, SHFL>(out, in, u, g, am, imass, am3, aux, om, bid, partials);
 }
 
 // Shamir kernel with K site groups per block (sites per CTA): blockDim = (Ls, K x the
@@ -219,7 +160,7 @@ __global__ void __launch_bounds__(128 * K, MINB)
   if (SHFL || live) {  // with SHFL every lane takes part (spare rows on a clamped site)
     const int st = live ? site : g.v3 - 1;
     C acc[4];
-    apply_site<S, 0, DAG, SHFL>(in, u, g, s, st, am, imass, am3, acc);
+    shamir_site<S, DAG, SHFL>(in, u, g, s, st, am, imass, am3, acc);
     if (live) {
 #pragma unroll
       for (int d = 0; d < 4; d++) epi_element<S, EPI, false>(out, aux, om, sidx32(g, s, site, d), acc[d], racc);
@@ -921,7 +862,7 @@ bool tile_maps(const Geom& g, const double2* in, const double2* u, tile::Maps* m
 // arithmetic type, with a partial of |rv|^2 (coef_e = coef[e * coef_stride], the entry's
 // own CG scalar; out is not written)
 template <class S, int KER, bool DAG, int EPI>
-__global__ void __launch_bounds__(256, KER == 0 ? 4 : 1)
+__global__ void __launch_bounds__(256, KER == 0 ? 4 : 2)
     k_dslash_batch(S* __restrict__ out, const S* __restrict__ in, const typename Sto<S>::C* __restrict__ u,
                    const BatchEntry* __restrict__ tab, int nent, int total_blocks, float am, int imass, float am3,
                    const int* skip, const S* __restrict__ aux, double* __restrict__ partials,
@@ -942,9 +883,16 @@ __global__ void __launch_bounds__(256, KER == 0 ? 4 : 1)
     const int sub = threadIdx.x / g.ls;
     const int site = (wb - E.blk0) * E.spb + sub;
     double racc = 0.0;
-    if (sub < E.spb && site < g.v3) {
-      C acc[4];
-      apply_site<S, KER, DAG>(in + E.off, u + E.uoff, g, s, site, am, imass, am3, acc);
+    const bool live = sub < E.spb && site < g.v3;
+    C acc[4];
+    if constexpr (KER == 1) {
+      extern __shared__ __align__(16) unsigned char wsm[];
+      wilson_exchange<S, false, DAG, 256>(in + E.off, u + E.uoff, g, s, site, live, threadIdx.x, am, imass, am3,
+                                          nullptr, reinterpret_cast<C*>(wsm), acc);
+    } else {
+      if (live) shamir_site<S, DAG, false>(in + E.off, u + E.uoff, g, s, site, am, imass, am3, acc);
+    }
+    if (live) {
       if (EPI == 4) {
         const R a = (R)coef[(size_t)lo * coef_stride];
         C* r = rv + E.off;
@@ -965,6 +913,7 @@ __global__ void __launch_bounds__(256, KER == 0 ? 4 : 1)
       }
     }
     if (EPI != 0) block_partial(racc, partials + wb);
+    else if (KER == 1) __syncthreads();  // the exchange buffer is free for the next work block
   }
 }
 
@@ -985,11 +934,8 @@ int device_sms() {
 }
 
 namespace {
-int stencil_threads(const Geom& g, int kernel) {
-  const int nt = kernel == 0 ? 128 : 256;
-  return g.ls <= nt ? nt : 1024;
-}
-bool stencil_shfl(const Geom& g, int kernel) { return kernel == 0 && g.ls <= 32 && (g.ls & (g.ls - 1)) == 0; }
+int stencil_threads(const Geom& g) { return g.ls <= 128 ? 128 : 1024; }
+bool stencil_shfl(const Geom& g) { return g.ls <= 32 && (g.ls & (g.ls - 1)) == 0; }
 // THR_TILE=1 in the environment puts the FP64 Shamir stencil on the staged-tile
 // kernel where the lattice allows it.  It is off by default: on B200 it measured
 // 51-54 us per launch in the 32^2x32, Ls 32 multishift solve against k_dslash's
@@ -1024,8 +970,8 @@ unsigned stencil_parts(const Geom& g, int kernel, bool fp64) {
   return fp64 && tile_ok(g, kernel) ? tile_grid(g) : stencil_grid(g, kernel);
 }
 
-dim3 stencil_block(const Geom& g, int kernel) {
-  int spb = stencil_threads(g, kernel) / g.ls;
+dim3 stencil_block(const Geom& g, int) {
+  int spb = stencil_threads(g) / g.ls;
   if (spb < 1) spb = 1;
   return dim3(g.ls, spb, 1);
 }
@@ -1040,7 +986,7 @@ unsigned stencil_grid(const Geom& g, int kernel) {
 // ---------------------------------------------------------------- autotuner
 // For the stencils in FP64 and FP32 storage the register budget (blocks per SM
 // the compiler may assume: 8, 7 or 6 for the Shamir kernel's 128-thread blocks,
-// 4, 3 or 2 for the Wilson kernel's 256-thread blocks) is tuned per (storage,
+// 6, 4 or 8 for the Wilson and overlap kernel's) is tuned per (storage,
 // kernel, M or M^dagger, epilogue, lattice, layout, device) on first use:
 // each candidate runs 1 + 3 times on the call's own fields (the launches are
 // idempotent: out and partials are overwritten), the fastest is kept for the
@@ -1052,7 +998,7 @@ unsigned stencil_grid(const Geom& g, int kernel) {
 // output element with the same operations
 // and sums the partials over the same site groups in the same order, so the
 // results do not change.  THR_TUNE=0 in the environment keeps the defaults
-// (8, 4); THR_TUNE=<n> runs candidate n wherever it is one.  Launches made
+// (8, 6); THR_TUNE=<n> runs candidate n wherever it is one.  Launches made
 // while the stream is being captured into a graph use the default until a
 // tuned value exists.
 namespace {
@@ -1067,8 +1013,7 @@ constexpr int kG2Code = 200;
 // same kernel reading the fifth-dimension neighbours from memory instead (the same
 // values, so the same bits): candidates kNoShflCode + 8, kNoShflCode + 6
 constexpr int kNoShflCode = 100;
-constexpr int kTuneWilson[3] = {4, 3, 2};
-constexpr int kTuneOverlap[3] = {4, 3, 1};  // k_odslash's 256-thread blocks
+constexpr int kTuneWilson[3] = {6, 4, 8};  // k_wilson's 128-thread blocks, Wilson and overlap
 constexpr int kMaxCand = 10;
 struct TuneKey {
   int dev, sid, ker, dag, epi, lx, ly, lt, ls, layout;
@@ -1157,6 +1102,60 @@ int tune_lookup(const TuneKey& key, const int* cand) {
   return it != g_tune.end() ? it->second.pick : cand[0];
 }
 
+// Wilson (OV false) and overlap (OV true) stencils, epilogues as launch_dslash_mode's.
+// 128-thread blocks for Ls <= 128 (register budget tuned like the Shamir kernel's), else one
+// block of up to 1024 threads per group of sites.  The exchange buffer is dynamic shared
+// memory: 8 (M) or 4 (M^dagger) values per thread.
+template <class S, bool OV>
+int launch_wilson(const Geom& g, bool dag, S* out, const S* in, const typename Sto<S>::C* u, float am, int imass,
+                  float am3, const double* zc, cudaStream_t st, const int* skip, const S* aux, const double* coef,
+                  double* partials, int e, int rev, bool may_tune, bool pdl) {
+  const dim3 blk = stencil_block(g, 1);
+  const dim3 grd(stencil_grid(g, 1));
+  const int nt = stencil_threads(g);
+  int dev = 0;
+  cudaGetDevice(&dev);
+#define THR_W(D, E, N, MB)                                                                                       \
+  do {                                                                                                           \
+    constexpr size_t bytes = (size_t)(D ? 4 : 8) * N * sizeof(typename Sto<S>::C);                               \
+    auto kern = k_wilson<S, OV, D, E, N, MB>;                                                                    \
+    if (bytes > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);  \
+    launch_k(kern, grd, blk, bytes, st, pdl, out, in, u, g, am, imass, am3, zc, skip, aux, coef, partials, rev); \
+  } while (0)
+#define THR_WE(D, N, MB)                             \
+  do {                                               \
+    if constexpr (OV) {                              \
+      THR_W(D, 0, N, MB);                            \
+    } else {                                         \
+      if (e == 1) THR_W(D, 1, N, MB);                \
+      else if (e == 2) THR_W(D, 2, N, MB);           \
+      else if (e == 3) THR_W(D, 3, N, MB);           \
+      else THR_W(D, 0, N, MB);                       \
+    }                                                \
+  } while (0)
+#define THR_WD(N, MB)               \
+  do {                              \
+    if (dag) THR_WE(true, N, MB);   \
+    else THR_WE(false, N, MB);      \
+  } while (0)
+  auto launch = [&](int minb) {
+    if (nt != 128) THR_WD(1024, 1);
+    else if (minb == 8) THR_WD(128, 8);
+    else if (minb == 4) THR_WD(128, 4);
+    else THR_WD(128, 6);
+  };
+#undef THR_WD
+#undef THR_WE
+#undef THR_W
+  int minb = kTuneWilson[0];
+  if (storage_id<S>() < 2 && nt == 128) {
+    const TuneKey key{dev, storage_id<S>(), OV ? 2 : 1, dag ? 1 : 0, e, g.lx, g.ly, g.lt, g.ls, g.layout};
+    minb = may_tune ? tune_pick(key, kTuneWilson, 3, st, launch) : tune_lookup(key, kTuneWilson);
+  }
+  launch(minb);
+  return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
+}
+
 // epi: 0 none, 1 out = aux + (*coef) M in with |out|^2 per block, 2 |out|^2 per block
 // may_tune false: no timing launches and no events (a budget tuned earlier is still used)
 template <class S>
@@ -1206,31 +1205,33 @@ int launch_dslash_mode(const Geom& g, int kernel, bool dag, S* out, const S* in,
 #undef THR_T
     return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
   }
+  if (kernel == 1)
+    return launch_wilson<S, false>(g, dag, out, in, u, am, imass, am3, nullptr, st, skip, aux, coef, partials, e, rev,
+                                   may_tune, pdl);
   const dim3 blk = stencil_block(g, kernel);
   const dim3 grd(stencil_grid(g, kernel));
-  const int nt = stencil_threads(g, kernel);
-  const bool shfl = stencil_shfl(g, kernel);
-#define THR_L(K, D, E, N, SH, MB)                                                                           \
-  launch_k(k_dslash<S, K, D, E, N, SH, MB>, grd, blk, 0, st, pdl, out, in, u, g, am, imass, am3, skip, aux, coef, \
+  const int nt = stencil_threads(g);
+  const bool shfl = stencil_shfl(g);
+#define THR_L(D, E, N, SH, MB)                                                                           \
+  launch_k(k_dslash<S, D, E, N, SH, MB>, grd, blk, 0, st, pdl, out, in, u, g, am, imass, am3, skip, aux, coef, \
            partials, rev)
-#define THR_E(K, D, N, SH, MB)                 \
-  do {                                         \
-    if (e == 1) THR_L(K, D, 1, N, SH, MB);     \
-    else if (e == 2) THR_L(K, D, 2, N, SH, MB); \
-    else if (e == 3) THR_L(K, D, 3, N, SH, MB); \
-    else THR_L(K, D, 0, N, SH, MB);            \
+#define THR_E(D, N, SH, MB)                 \
+  do {                                      \
+    if (e == 1) THR_L(D, 1, N, SH, MB);     \
+    else if (e == 2) THR_L(D, 2, N, SH, MB); \
+    else if (e == 3) THR_L(D, 3, N, SH, MB); \
+    else THR_L(D, 0, N, SH, MB);            \
   } while (0)
-#define THR_D(K, N, SH, MB)                        \
-  do {                                             \
-    if (dag) THR_E(K, true, N, SH, MB);            \
-    else THR_E(K, false, N, SH, MB);               \
+#define THR_D(N, SH, MB)                        \
+  do {                                          \
+    if (dag) THR_E(true, N, SH, MB);            \
+    else THR_E(false, N, SH, MB);               \
   } while (0)
   // FP32 Shamir with even Ls: two s per thread (k_dslash_pair), same grid
-  const bool pair = storage_id<S>() == 1 && kernel == 0 && nt == 128 && g.ls % 2 == 0;
+  const bool pair = storage_id<S>() == 1 && nt == 128 && g.ls % 2 == 0;
 
   // the register budget (resident blocks per SM) of the common configurations is
   // tuned: Shamir 128-thread blocks {8, 7, 6} (pair kernel: 64-thread blocks {16, 14, 12}),
-  // Wilson 256-thread blocks {2, 1}
   auto launch = [&](int minb) {
     if (pair) {
       const dim3 pblk(g.ls / 2, blk.y, 1);
@@ -1262,23 +1263,11 @@ int launch_dslash_mode(const Geom& g, int kernel, bool dag, S* out, const S* in,
 #undef THR_P
       return;
     }
-    if (kernel == 1) {
-      // Ls a power of two <= 32: the fifth-dimension slices from warp shuffles
-      const bool wshfl = g.ls <= 32 && (g.ls & (g.ls - 1)) == 0;
-      if (nt != 256) THR_D(1, 1024, false, 1);
-      else if (minb == kNoShflCode + 4) THR_D(1, 256, false, 4);  // the slices from memory
-      else if (minb == kNoShflCode + 2) THR_D(1, 256, false, 2);
-      else if (wshfl && minb == 4) THR_D(1, 256, true, 4);
-      else if (wshfl && minb == 3) THR_D(1, 256, true, 3);
-      else if (wshfl) THR_D(1, 256, true, 2);
-      else if (minb == 4) THR_D(1, 256, false, 4);
-      else if (minb == 3) THR_D(1, 256, false, 3);
-      else THR_D(1, 256, false, 2);
-    } else if (nt != 128) {
-      THR_D(0, 1024, false, 1);
+    if (nt != 128) {
+      THR_D(1024, false, 1);
     } else if (minb > kNoShflCode && minb < kG2Code) {
-      if (minb == kNoShflCode + 8) THR_D(0, 128, false, 8);
-      else THR_D(0, 128, false, 6);
+      if (minb == kNoShflCode + 8) THR_D(128, false, 8);
+      else THR_D(128, false, 6);
     } else if (minb > kG2Code) {
       if constexpr (storage_id<S>() == 0) {
         const int K = (minb - kG2Code) / 10;
@@ -1338,19 +1327,19 @@ int launch_dslash_mode(const Geom& g, int kernel, bool dag, S* out, const S* in,
 #undef THR_S
       }
     } else if (shfl) {
-      if (minb == 8) THR_D(0, 128, true, 8);
-      else if (minb == 7) THR_D(0, 128, true, 7);
-      else THR_D(0, 128, true, 6);
+      if (minb == 8) THR_D(128, true, 8);
+      else if (minb == 7) THR_D(128, true, 7);
+      else THR_D(128, true, 6);
     } else {
-      if (minb == 8) THR_D(0, 128, false, 8);
-      else if (minb == 7) THR_D(0, 128, false, 7);
-      else THR_D(0, 128, false, 6);
+      if (minb == 8) THR_D(128, false, 8);
+      else if (minb == 7) THR_D(128, false, 7);
+      else THR_D(128, false, 6);
     }
   };
-  const bool tunable = storage_id<S>() < 2 && nt == (kernel == 0 ? 128 : 256);
+  const bool tunable = storage_id<S>() < 2 && nt == 128;
   // FP64 Shamir, 128-thread blocks: the four-threads-per-site kernel; where a block is
   // whole warps also the two-group blocks
-  const bool split_ok = kernel == 0 && storage_id<S>() == 0;
+  const bool split_ok = storage_id<S>() == 0;
   const bool g2_ok = split_ok && (blk.x * blk.y) % 32 == 0;
   int cand64[kMaxCand] = {8, 7, 6};
   int ncand = 3;
@@ -1367,15 +1356,7 @@ int launch_dslash_mode(const Geom& g, int kernel, bool dag, S* out, const S* in,
       cand64[ncand++] = kNoShflCode + 6;
     }
   }
-  // Wilson with Ls a power of two <= 32: the shuffle kernel's budgets, and the same kernel
-  // reading the fifth-dimension slices from memory (the same values and bits)
-  int candw[kMaxCand] = {kTuneWilson[0], kTuneWilson[1], kTuneWilson[2]};
-  if (kernel == 1 && g.ls <= 32 && (g.ls & (g.ls - 1)) == 0) {
-    candw[3] = kNoShflCode + 4;
-    candw[4] = kNoShflCode + 2;
-    ncand = 5;
-  }
-  const int* cand = kernel == 0 ? (split_ok ? cand64 : kTuneShamir) : candw;
+  const int* cand = split_ok ? cand64 : kTuneShamir;
   int minb = cand[0];
   if (tunable) {
     int dev = 0;
@@ -1433,29 +1414,8 @@ int launch_odslash(const Geom& g, bool dag, double2* out, const double2* in, con
   if (g.ls > 1024) return THR_ERR_BADSHAPE;
   if (4ULL * (unsigned long long)g.v5 >= (1ULL << 32)) return THR_ERR_BADSHAPE;  // 32-bit element offsets
   if (imass != 1 && imass != 3) return THR_ERR_UNSUPPORTED;  // measure_OWilson.F90:66-83
-  const dim3 blk = stencil_block(g, 1);
-  const dim3 grd(stencil_grid(g, 1));
-  // register budget (resident 256-thread blocks per SM) tuned per lattice and direction like
-  // the other stencils: 4 and 3 win on large lattices, 1 on small ones
-#define THR_O(D, MB) k_odslash<D, MB><<<grd, blk, 0, st>>>(out, in, u, g, am, imass, am3, zc, skip)
-  auto launch = [&](int mb) {
-    if (dag) {
-      if (mb == 4) THR_O(true, 4);
-      else if (mb == 3) THR_O(true, 3);
-      else THR_O(true, 1);
-    } else {
-      if (mb == 4) THR_O(false, 4);
-      else if (mb == 3) THR_O(false, 3);
-      else THR_O(false, 1);
-    }
-  };
-#undef THR_O
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const int mb = tune_pick(TuneKey{dev, 0, 2, dag ? 1 : 0, 0, g.lx, g.ly, g.lt, g.ls, g.layout}, kTuneOverlap, 3, st,
-                           launch);
-  launch(mb);
-  return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
+  return launch_wilson<double2, true>(g, dag, out, in, u, am, imass, am3, zc, st, skip, nullptr, nullptr, nullptr, 0, 0,
+                                      true, false);
 }
 
 // The persistent batch stencil's grid (resident blocks per SM) is tuned like the register
@@ -1471,7 +1431,8 @@ int launch_dslash_batch(const BatchTable& b, int kernel, bool dag, S* out, const
   auto launch = [&](int per_sm) {
     const int g = grid > 0 ? grid : std::min(b.total_blocks, device_sms() * per_sm);
 #define THR_L(K, D, E)                                                                                          \
-  k_dslash_batch<S, K, D, E><<<g, 256, 0, st>>>(out, in, u, b.dev, b.nent, b.total_blocks, am, imass, am3, skip, \
+  k_dslash_batch<S, K, D, E><<<g, 256, K ? (D ? 4 : 8) * 256 * sizeof(typename Sto<S>::C) : 0, st>>>(             \
+      out, in, u, b.dev, b.nent, b.total_blocks, am, imass, am3, skip,                                          \
                                                 aux, partials, nullptr, nullptr, 0)
     if (kernel == 1) {
       if (dag) { if (epi) THR_L(1, true, 1); else THR_L(1, true, 0); }
@@ -1505,7 +1466,8 @@ int launch_dslash_batch_fused(const BatchTable& b, int kernel, bool dag, int epi
   auto launch = [&](int per_sm) {
     const int g = grid > 0 ? grid : std::min(b.total_blocks, device_sms() * per_sm);
 #define THR_L(K, D, E)                                                                                          \
-  k_dslash_batch<S, K, D, E><<<g, 256, 0, st>>>(out, in, u, b.dev, b.nent, b.total_blocks, am, imass, am3, skip, \
+  k_dslash_batch<S, K, D, E><<<g, 256, K ? (D ? 4 : 8) * 256 * sizeof(typename Sto<S>::C) : 0, st>>>(             \
+      out, in, u, b.dev, b.nent, b.total_blocks, am, imass, am3, skip,                                          \
                                                 nullptr, partials, rv, coef, coef_stride)
     if (kernel == 1) {
       if (dag) { if (epi == 4) THR_L(1, true, 4); else THR_L(1, true, 2); }

@@ -175,135 +175,6 @@ __device__ __forceinline__ void shamir_site(const S* __restrict__ in, const type
   }
 }
 
-// ---------------------------------------------------------------- Wilson
-// a complex value from lane `src` of this lane's Ls-wide segment (every lane calls it)
-template <class C>
-__device__ __forceinline__ C seg_shfl(C v, int src, int Ls) {
-  return mk(__shfl_sync(0xffffffffu, v.x, src, Ls), __shfl_sync(0xffffffffu, v.y, src, Ls));
-}
-
-// Q(s) components for the forward operator at (s, site).  SHFL: the slices s-1, s+1 and
-// the walls' R(Ls), R(1) come from the lanes of the same site (blockDim.x = Ls a power of
-// two <= 32; every lane must call this): the same values, one load per spin instead of three.
-template <class S, bool COH, bool SHFL = false>
-__device__ __forceinline__ void wilson_q(const SpinorView<S, COH>& Rv, int s, int site, int Ls,
-                                         typename Sto<S>::C c1, typename Sto<S>::C c2,
-                                         typename Sto<S>::C* q) {
-  using C = typename Sto<S>::C;
-  C r[4];
-#pragma unroll
-  for (int d = 0; d < 4; d++) r[d] = Rv(s, site, d);
-  if (SHFL) {
-#pragma unroll
-    for (int d = 0; d < 2; d++) {
-      const C prv = seg_shfl(r[d], s > 0 ? s - 1 : Ls - 1, Ls);
-      q[d] = (s > 0) ? r[d] + prv : r[d] + cmul(c1, prv);
-    }
-#pragma unroll
-    for (int d = 2; d < 4; d++) {
-      const C nxt = seg_shfl(r[d], s < Ls - 1 ? s + 1 : 0, Ls);
-      q[d] = (s < Ls - 1) ? r[d] + nxt : r[d] + cmul(c2, nxt);
-    }
-    return;
-  }
-  // P+ (spins 0,1) from s-1, wall: c1 * R(Ls)
-#pragma unroll
-  for (int d = 0; d < 2; d++) q[d] = (s > 0) ? r[d] + Rv(s - 1, site, d) : r[d] + cmul(c1, Rv(Ls - 1, site, d));
-  // P- (spins 2,3) from s+1, wall: c2 * R(1)
-#pragma unroll
-  for (int d = 2; d < 4; d++) q[d] = (s < Ls - 1) ? r[d] + Rv(s + 1, site, d) : r[d] + cmul(c2, Rv(0, site, d));
-}
-
-template <class S, bool DAG, bool COH = false, bool SHFL = false>
-__device__ __forceinline__ void wilson_site(const S* __restrict__ in, const typename Sto<S>::C* __restrict__ u,
-                                            const Geom& g, int s, int site, float am, int imass, float am3,
-                                            typename Sto<S>::C* res) {
-  using R = typename Sto<S>::R;
-  using C = typename Sto<S>::C;
-  int x, y, t;
-  site_coords(g, site, x, y, t);
-  const Nbr nb = neighbours(g, site, x, y, t);
-  SpinorView<S, COH> Rv{in, g};
-  const int Ls = g.ls;
-  const R a = (R)am;
-  const R dgw = (R)(3.0f + (-am3));  // DWilson(…, -am3) diagonal: dirac.F90:191, :505
-  if (!DAG) {
-    // c1 = -am | -i am  (dirac.F90:274-278),  c2 = -am | +i am  (dirac.F90:287-291)
-    const C c1 = imass == 1 ? mk(-a, R(0)) : mk(R(0), -a);
-    const C c2 = imass == 1 ? mk(-a, R(0)) : mk(R(0), a);
-    C q[4];
-    wilson_q<S, COH, SHFL>(Rv, s, site, Ls, c1, c2, q);
-#pragma unroll
-    for (int d = 0; d < 4; d++) res[d] = (dgw - R(1)) * q[d] + R(2) * Rv(s, site, d);
-    // D_W hops of Q (dirac.F90:197-217), spin-projected as in the Shamir kernel
-#pragma unroll
-    for (int mu = 0; mu < 3; mu++) {
-      const C U = __ldg(u + (size_t)mu * g.v3 + site);
-      const C Ub = cconj(__ldg(u + (size_t)mu * g.v3 + nb.b[mu]));
-      C q[4];
-      wilson_q<S, COH, SHFL>(Rv, s, nb.f[mu], Ls, c1, c2, q);
-      hop_projected<C, R>(mu, true, U, q, res);
-      wilson_q<S, COH, SHFL>(Rv, s, nb.b[mu], Ls, c1, c2, q);
-      hop_projected<C, R>(mu, false, Ub, q, res);
-    }
-  } else {
-    // z = -am | -i am (upper right, dirac.F90:602-606); z' = -am | +i am (lower left, :615-619)
-    const C z = imass == 1 ? mk(-a, R(0)) : mk(R(0), -a);
-    const C zp = imass == 1 ? mk(-a, R(0)) : mk(R(0), a);
-    // half 0: output spins 0,1 use Qp = R(s) + R(s+1) | z' R(1); half 1: spins 2,3 use Qm = R(s) + R(s-1) | z R(Ls).
-    // One pass over the neighbours serves both halves: R(s) and the two partner slices are loaded
-    // once per site (each output element gets the same operations in the same order as half by half)
-    const bool in0 = s < Ls - 1, in1 = s > 0;
-    const int sp0 = in0 ? s + 1 : 0, sp1 = in1 ? s - 1 : Ls - 1;
-    auto qpair = [&](int st, C* q0, C* q1) {
-#pragma unroll
-      for (int d = 0; d < 4; d++) {
-        const C r = Rv(s, st, d);
-        const C a0 = SHFL ? seg_shfl(r, sp0, Ls) : Rv(sp0, st, d);
-        const C a1 = SHFL ? seg_shfl(r, sp1, Ls) : Rv(sp1, st, d);
-        q0[d] = in0 ? r + a0 : r + cmul(zp, a0);
-        q1[d] = in1 ? r + a1 : r + cmul(z, a1);
-      }
-    };
-    {
-      C q0[4], q1[4];
-      qpair(site, q0, q1);
-#pragma unroll
-      for (int k = 0; k < 2; k++) {
-        res[k] = (dgw - R(1)) * q0[k] + R(2) * Rv(s, site, k);
-        res[2 + k] = (dgw - R(1)) * q1[2 + k] + R(2) * Rv(s, site, 2 + k);
-      }
-    }
-    // D_W^dagger hops (dirac.F90:511-531): -1/2 W [q(d) +- 2gamma(mu,d) q(gin)], each half's
-    // output spins from its own Q
-#pragma unroll
-    for (int mu = 0; mu < 3; mu++) {
-      const C U = __ldg(u + (size_t)mu * g.v3 + site);
-      const C Ub = cconj(__ldg(u + (size_t)mu * g.v3 + nb.b[mu]));
-#pragma unroll
-      for (int dir = 0; dir < 2; dir++) {
-        C q0[4], q1[4];
-        qpair(dir == 0 ? nb.f[mu] : nb.b[mu], q0, q1);
-        const C W = dir == 0 ? U : Ub;
-#pragma unroll
-        for (int d = 0; d < 4; d++) {
-          const C* q = d < 2 ? q0 : q1;
-          const GammaEntry ge = gamma_entry(mu, d);
-          const C gq = gp(ge, q[ge.gin]);
-          res[d] = res[d] - R(0.5) * cmul(W, dir == 0 ? q[d] + gq : q[d] - gq);
-        }
-      }
-    }
-  }
-}
-
-template <class S, int KER, bool DAG, bool SHFL = false, bool COH = false>
-__device__ __forceinline__ void apply_site(const S* in, const typename Sto<S>::C* u, const Geom& g, int s, int site,
-                                           float am, int imass, float am3, typename Sto<S>::C* acc) {
-  if (KER == 0) shamir_site<S, DAG, SHFL, COH>(in, u, g, s, site, am, imass, am3, acc);
-  else wilson_site<S, DAG, COH, SHFL>(in, u, g, s, site, am, imass, am3, acc);
-}
-
 // One block's sites of the stencil with its epilogue (blockDim = (Ls, sites per
 // block), NT threads at most; the block's sites are bid * blockDim.y + threadIdx.y).
 // Epilogues (EPI): 0 store out = M in; 2 also one FP64 partial of |out|^2 into
@@ -353,7 +224,7 @@ __device__ __forceinline__ void block_partial_sum(double racc, double* __restric
   }
 }
 
-template <class S, int KER, bool DAG, int EPI, int NT, bool SHFL, bool COH = false>
+template <class S, bool DAG, int EPI, int NT, bool SHFL, bool COH = false>
 __device__ __forceinline__ void dslash_block(S* __restrict__ out, const S* __restrict__ in,
                                              const typename Sto<S>::C* __restrict__ u, const Geom& g, float am,
                                              int imass, float am3, const S* __restrict__ aux,
@@ -366,7 +237,7 @@ __device__ __forceinline__ void dslash_block(S* __restrict__ out, const S* __res
   if (SHFL || live) {  // with SHFL every lane takes part (the last block's spare rows on a clamped site)
     const int st = live ? site : g.v3 - 1;
     C acc[4];
-    apply_site<S, KER, DAG, SHFL, COH>(in, u, g, s, st, am, imass, am3, acc);
+    shamir_site<S, DAG, SHFL, COH>(in, u, g, s, st, am, imass, am3, acc);
     if (live) {
 #pragma unroll
       for (int d = 0; d < 4; d++) epi_element<S, EPI, COH>(out, aux, om, sidx32(g, s, site, d), acc[d], racc);
@@ -377,7 +248,7 @@ __device__ __forceinline__ void dslash_block(S* __restrict__ out, const S* __res
 
 // the stencil part of dslash_block alone: the thread's M in (acc); spare rows compute a
 // clamped site (SHFL) or nothing
-template <class S, int KER, bool DAG, bool SHFL, bool COH = false>
+template <class S, bool DAG, bool SHFL, bool COH = false>
 __device__ __forceinline__ void block_sites(const S* __restrict__ in, const typename Sto<S>::C* __restrict__ u,
                                             const Geom& g, float am, int imass, float am3, int bid,
                                             typename Sto<S>::C* acc) {
@@ -386,7 +257,135 @@ __device__ __forceinline__ void block_sites(const S* __restrict__ in, const type
   const bool live = site < g.v3;
   if (SHFL || live) {
     const int st = live ? site : g.v3 - 1;
-    apply_site<S, KER, DAG, SHFL, COH>(in, u, g, s, st, am, imass, am3, acc);
+    shamir_site<S, DAG, SHFL, COH>(in, u, g, s, st, am, imass, am3, acc);
+  }
+}
+
+// ---------------------------------------------------------------- Wilson, overlap
+// The hops are diagonal in s and the links do not depend on s, so the 3D operator D_W and
+// the s-combinations of the slices commute: each thread applies the six hops to its own
+// slice R(s) only -- four loads per neighbour site, as the Shamir kernel -- and the
+// neighbouring slices' results are combined afterwards through shared memory.
+//   M:     Q(s) = R(s) + wA P+ R(s-1) + wB P- R(s+1).  A = the hops of the upper spins of
+//          R(s) (to all four output spins), B those of the lower spins; then
+//          D_W Q(s) = [A + B](s) + wA A(s-1) + wB B(s+1).
+//   M^dag: the output's upper spins take D_W^dag (R(s) + w R(s+1)), the lower ones
+//          D_W^dag (R(s) + w R(s-1)): one spin-projected hop pass, then one exchange.
+// (Building Q at every neighbour first costs 8 to 12 loads per neighbour site.)  The
+// overlap operator is the same with slice s's D_W scaled by its coefficient c[s].
+
+// hops of the upper (A) and lower (B) spins of r apart, without the common factor -1/2
+template <class C>
+__device__ __forceinline__ void hop_halves(int mu, bool plus, C W, const C* r, C* A, C* B) {
+#pragma unroll
+  for (int d = 0; d < 4; d++) {
+    const C T = cmul(W, r[d]);
+    const int gi = gamma_entry(mu, d).gin;
+    const C gt = gp(gamma_entry(mu, gi), T);
+    C* X = d < 2 ? A : B;
+    X[d] = X[d] + T;
+    X[gi] = plus ? X[gi] - gt : X[gi] + gt;
+  }
+}
+
+// One 5D site of the Wilson (OV false) or overlap (OV true) operator.  Every thread of the
+// block calls it (live false: a thread without a site); ex: NT x (DAG ? 4 : 8) values in
+// shared memory, read by nobody once every thread has returned from a __syncthreads().
+// tid - s .. tid - s + Ls - 1 are the threads of this thread's site.
+template <class S, bool OV, bool DAG, int NT>
+__device__ __forceinline__ void wilson_exchange(const S* __restrict__ in, const typename Sto<S>::C* __restrict__ u,
+                                                const Geom& g, int s, int site, bool live, int tid, float am,
+                                                int imass, float am3, const double* __restrict__ zc,
+                                                typename Sto<S>::C* ex, typename Sto<S>::C* res) {
+  using R = typename Sto<S>::R;
+  using C = typename Sto<S>::C;
+  const int Ls = g.ls;
+  const R a = (R)am;
+  const R dgw = (R)(3.0f + (-am3));  // DWilson(..., -am3) diagonal: dirac.F90:191, :505
+  C r[4], A[4], B[4];
+  const S* pl[4];
+#pragma unroll
+  for (int d = 0; d < 4; d++) pl[d] = in + (size_t)d * (size_t)g.v5;
+  if (live) {
+    int x, y, t;
+    site_coords(g, site, x, y, t);
+    const Nbr nb = neighbours(g, site, x, y, t);
+    const unsigned i0 = (unsigned)s + (unsigned)Ls * (unsigned)site;
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+      r[d] = Sto<S>::ld(pl[d], i0);
+      A[d] = B[d] = mk(R(0), R(0));
+    }
+    if (DAG) {
+#pragma unroll
+      for (int d = 0; d < 4; d++) A[d] = (OV ? dgw : dgw - R(1)) * r[d];
+    }
+#pragma unroll
+    for (int mu = 0; mu < 3; mu++) {
+#pragma unroll
+      for (int dir = 0; dir < 2; dir++) {
+        const int ns = dir == 0 ? nb.f[mu] : nb.b[mu];
+        const C W = dir == 0 ? __ldg(u + (size_t)mu * g.v3 + site) : cconj(__ldg(u + (size_t)mu * g.v3 + nb.b[mu]));
+        const unsigned i = (unsigned)s + (unsigned)Ls * (unsigned)ns;
+        C q[4];
+#pragma unroll
+        for (int d = 0; d < 4; d++) q[d] = Sto<S>::ld(pl[d], i);
+        if (DAG) hop_projected<C, R>(mu, dir != 0, W, q, A);
+        else hop_halves<C>(mu, dir == 0, W, q, A, B);
+      }
+    }
+    const R cs = OV ? (R)__ldg(zc + s) : R(1);
+    if (DAG) {
+#pragma unroll
+      for (int d = 0; d < 4; d++) {
+        if (OV) A[d] = cs * A[d] - r[d];
+        ex[d * NT + tid] = A[d];
+      }
+    } else {
+      const R dd = OV ? dgw : dgw - R(1);
+#pragma unroll
+      for (int d = 0; d < 4; d++) {
+        A[d] = (d < 2) ? dd * r[d] - R(0.5) * A[d] : R(-0.5) * A[d];
+        B[d] = (d < 2) ? R(-0.5) * B[d] : dd * r[d] - R(0.5) * B[d];
+        ex[d * NT + tid] = A[d];
+        ex[(4 + d) * NT + tid] = B[d];
+      }
+    }
+  }
+  __syncthreads();
+  if (!live) return;
+  const bool inp = s > 0, inn = s < Ls - 1;
+  const int tp = inp ? tid - 1 : tid + Ls - 1, tn = inn ? tid + 1 : tid - (Ls - 1);
+  const R sg = OV ? R(-1) : R(1);  // the overlap module's imass 3 walls have the opposite sign
+  // wall factors: wp on the slice before (s = 0: the last one), wn on the slice after
+  // M: c1, c2 (dirac.F90:274-278, :287-291); M^dag: z, z' (:602-606, :615-619): the same values;
+  // overlap: m1, m2 (measure_OWilson.F90:66-83) and z1, z2 (:139-157)
+  const C wp = imass == 1 ? mk(-a, R(0)) : mk(R(0), -sg * a);
+  const C wn = imass == 1 ? mk(-a, R(0)) : mk(R(0), sg * a);
+  if (DAG) {
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+      const bool lo = d < 2;  // spins 0,1 from the slice after, 2,3 from the one before
+      const C v = ex[d * NT + (lo ? tn : tp)];
+      const C w = (lo ? inn : inp) ? v : cmul(lo ? wn : wp, v);
+      res[d] = A[d] + R(2) * r[d] + w;
+    }
+  } else {
+    const R cs = OV ? (R)__ldg(zc + s) : R(1);
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+      const C fa = ex[d * NT + tp], gb = ex[(4 + d) * NT + tn];
+      const C v = (A[d] + B[d]) + ((inp ? fa : cmul(wp, fa)) + (inn ? gb : cmul(wn, gb)));
+      if (OV) {
+        const bool lo = d < 2;
+        const C n = Sto<S>::ld(pl[d], (unsigned)Ls * (unsigned)site +
+                                          (unsigned)(lo ? (inp ? s - 1 : Ls - 1) : (inn ? s + 1 : 0)));
+        const C wr = (lo ? inp : inn) ? n : cmul(lo ? wp : wn, n);
+        res[d] = cs * v + r[d] - wr;
+      } else {
+        res[d] = v + R(2) * r[d];
+      }
+    }
   }
 }
 

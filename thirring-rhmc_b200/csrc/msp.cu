@@ -78,6 +78,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, int
 // The partials of a stencil pass, written by every block, are copied into shared memory
 // with cp.async (16 bytes each, through L2) right after the barrier, while the block
 // computes its next stencil pass; the sum waits for them only when its result is due.
+constexpr int kChainThreads = 128;     // the Shamir stencil's blocks
 constexpr int kChainMaxParts = 2048;  // partials one block stages (stencil site blocks)
 __device__ __forceinline__ void stage_partials(double* sp, const double* p, int n, int tid, int nthr) {
   const int n2 = (n + 1) & ~1;  // the arrays are padded to an even length
@@ -138,8 +139,8 @@ struct ChainArgs {
   unsigned extra;  // added to every barrier's target (the timeout test); 0 in use
 };
 
-template <int KER, int NT, bool SHFL>
-__global__ void __launch_bounds__(NT, 512 / NT) k_ms_chain(ChainArgs a) {
+template <bool SHFL>
+__global__ void __launch_bounds__(kChainThreads, 512 / kChainThreads) k_ms_chain(ChainArgs a) {
   using C = double2;
   __shared__ MsState st;
   __shared__ __align__(16) double sp[kChainMaxParts];
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_ms_chain(ChainArgs a) {
     bool first = true, stop = false;
     for (int t = blockIdx.x; t < a.np; t += gridDim.x) {
       C acc[4];
-      block_sites<double2, KER, false, SHFL, true>(rold, a.u, g, a.am, a.imass, a.am3, t, acc);
+      block_sites<double2, false, SHFL, true>(rold, a.u, g, a.am, a.imass, a.am3, t, acc);
       if (first) {
         first = false;
         if (lam_due) {
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_ms_chain(ChainArgs a) {
         for (int d = 0; d < 4; d++)
           epi_element<double2, 3, true>(hcur, hprev, st.gammag, sidx32(g, threadIdx.x, site, d), acc[d], racc);
       }
-      block_partial_sum<NT>(racc, a.pa, t);
+      block_partial_sum<kChainThreads>(racc, a.pa, t);
       __syncthreads();
     }
     if (stop) break;
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_ms_chain(ChainArgs a) {
     first = true;
     for (int t = blockIdx.x; t < a.np; t += gridDim.x) {
       C acc[4];
-      block_sites<double2, KER, true, SHFL, true>(hcur, a.u, g, a.am, a.imass, a.am3, t, acc);
+      block_sites<double2, true, SHFL, true>(hcur, a.u, g, a.am, a.imass, a.am3, t, acc);
       if (first) {
         first = false;
         ms_alpha_block(&st, rec, nstep, sum_staged(sp, a.np, tid, nthr, sh), tid);
@@ -229,7 +230,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_ms_chain(ChainArgs a) {
         for (int d = 0; d < 4; d++)
           epi_element<double2, 1, true>(rnew, rold, st.omega, sidx32(g, threadIdx.x, site, d), acc[d], racc);
       }
-      block_partial_sum<NT>(racc, a.pl, t);
+      block_partial_sum<kChainThreads>(racc, a.pl, t);
       __syncthreads();
     }
     target += gridDim.x;
@@ -290,7 +291,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_ms_chain(ChainArgs a) {
 }
 
 // co-resident blocks of a k_ms_chain instantiation on this device (cached per device)
-template <int KER, int NT, bool SHFL>
+template <bool SHFL>
 int chain_capacity() {
   constexpr int kDevs = 64;
   static std::atomic<int> cache[kDevs];
@@ -301,15 +302,15 @@ int chain_capacity() {
     if (v > 0) return v;
   }
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ms_chain<KER, NT, SHFL>, NT, 0) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ms_chain<SHFL>, kChainThreads, 0) != cudaSuccess) return 0;
   const int cap = occ * device_sms();
   if (dev < kDevs && cap > 0) cache[dev].store(cap, std::memory_order_relaxed);
   return cap;
 }
 
-template <int KER, int NT, bool SHFL>
+template <bool SHFL>
 int chain_launch(thr_ctx* c, const ChainArgs& a, dim3 blk, cudaStream_t st, bool dry) {
-  const int cap = chain_capacity<KER, NT, SHFL>();
+  const int cap = chain_capacity<SHFL>();
   if (cap <= 0) return THR_ERR_UNSUPPORTED;
   // auto (mode 1): only where every site block has its own resident block; forced (2): any size
   if (c->chain_mode == 1 && a.np > cap) return THR_ERR_UNSUPPORTED;
@@ -325,7 +326,7 @@ int chain_launch(thr_ctx* c, const ChainArgs& a, dim3 blk, cudaStream_t st, bool
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_ms_chain<KER, NT, SHFL>, a) == cudaSuccess ? THR_OK : THR_ERR_CUDA;
+  return cudaLaunchKernelEx(&cfg, k_ms_chain<SHFL>, a) == cudaSuccess ? THR_OK : THR_ERR_CUDA;
 }
 
 // THR_CHAIN_WAIT_TEST=1: every barrier expects one arrival more than the grid has, so
@@ -347,10 +348,10 @@ int ms_chain_batch(thr_ctx* c, MsState* ms, MsHist* rec, double2* ring, double2*
   const dim3 blk = stencil_block(g, kernel);
   const int nthr = (int)(blk.x * blk.y);
   const int np = (int)stencil_grid(g, kernel);
-  // the block shapes of the stencil kernels' common configurations (128-thread Shamir,
-  // 256-thread Wilson blocks) with at least nt / 32 - 1 whole warps (the sums' layout,
-  // sum_staged) and kMaxShift threads (the scalar steps)
-  const int nt = kernel == 0 ? 128 : 256;
+  if (kernel != 0) return THR_ERR_UNSUPPORTED;  // the Shamir stencil only
+  // the common block shape of the stencil kernel (128 threads) with at least nt / 32 - 1
+  // whole warps (the sums' layout, sum_staged) and kMaxShift threads (the scalar steps)
+  const int nt = kChainThreads;
   if (g.ls > nt || nthr > nt || nthr / 32 < nt / 32 - 1 || nthr < kMaxShift) return THR_ERR_UNSUPPORTED;
   const size_t npad = ((size_t)np + 1) & ~(size_t)1;  // pl 16-byte aligned, both arrays even
   if (np > kChainMaxParts || 2 * npad > c->nparts) return THR_ERR_UNSUPPORTED;
@@ -371,10 +372,9 @@ int ms_chain_batch(thr_ctx* c, MsState* ms, MsHist* rec, double2* ring, double2*
   a.half = half;
   a.bar = reinterpret_cast<unsigned*>(c->iscal + kIscalChainBar);
   a.extra = chain_extra();
-  const bool shfl = kernel == 0 && g.ls <= 32 && (g.ls & (g.ls - 1)) == 0;
-  if (kernel == 1) return chain_launch<1, 256, false>(c, a, blk, st, dry);
-  if (shfl) return chain_launch<0, 128, true>(c, a, blk, st, dry);
-  return chain_launch<0, 128, false>(c, a, blk, st, dry);
+  const bool shfl = g.ls <= 32 && (g.ls & (g.ls - 1)) == 0;
+  if (shfl) return chain_launch<true>(c, a, blk, st, dry);
+  return chain_launch<false>(c, a, blk, st, dry);
 }
 
 }  // namespace thr
