@@ -1,0 +1,31 @@
+"""Small-lattice solver iterations (the scalar steps inside the stencil kernels) against
+the kernel chain with one-block sums, which runs while kernel timings are sampled."""
+import numpy as np
+import pytest
+
+import oracle as O
+import thirring
+from helpers import rand_links, rand_spinor
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,layout", [((2, 2, 2, 8), 0), ((3, 5, 2, 33), 0), ((4, 6, 10, 20), 1),
+                                         ((12, 12, 12, 16), 0), ((16, 16, 12, 40), 0), ((16, 16, 14, 40), 1),
+                                         ((16, 16, 24, 40), 0)])
+@pytest.mark.parametrize("maxcg", [33, 150])
+def test_multishift_steps_bit_identical(dims, layout, maxcg):
+    """One block, idle threads, both site orders, up to 1024 partials and above (two per
+    thread of the sum), just under and over the largest lattice that takes the two-kernel
+    iteration; stopped inside a batch: the same bits and counts as the kernel chain."""
+    rng = np.random.default_rng(5)
+    L = O.lat(*dims)
+    u, inp = rand_links(L, rng), rand_spinor(L, rng)
+    aden, anum = np.array([1e-3, 0.05, 0.7, 30.0]), np.array([0.3, 0.5, 0.8, 2.0])
+    outs = []
+    with thirring.Lattice(*dims, layout=layout, ndiag=4) as G:
+        for stride in (0, 1 << 20):
+            G._L.thr_profile(G.h, stride, 1)
+            outs.append(G.multishift_solver(u, 0.05, 3, aden, anum, inp, 1e-7, maxcg))
+    (x, it, cgr), (xc, itc, cgrc) = outs
+    assert it == itc and np.array_equal(cgr, cgrc)
+    assert np.array_equal(x, xc)

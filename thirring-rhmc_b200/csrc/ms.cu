@@ -182,7 +182,7 @@ int ms_prepare_state(thr_ctx* c, MsState* h, int ndiagq, const double* aden, con
   h->hi = ndiagq - 1;
   h->maxcg = maxcg;
   h->res = res;
-  h->done = (maxcg <= 0);
+  h->done = h->halt = (maxcg <= 0);
   (void)c;
   return THR_OK;
 }

@@ -17,6 +17,10 @@ struct MsState {
   // mixed precision (batched solver): the FP64 phase ends once delta = |r|^2 falls
   // below switch_delta = switch_rel2 * |input|^2 (0: never)
   double switch_rel2, switch_delta;
+  // small lattices (steps.cu): delta before iteration j of a batch in dl[j & 1]; halt:
+  // `done` as the M step reads it
+  double dl[2];
+  int halt, pad;
   double zeta_i[kMaxShift], zeta_ii[kMaxShift], zeta_iii[kMaxShift];
   double omegas[kMaxShift], gammas[kMaxShift], correction[kMaxShift], aden[kMaxShift];
   int flags[kMaxShift], cg_returns[kMaxShift];

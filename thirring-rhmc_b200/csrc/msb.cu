@@ -27,6 +27,7 @@
 #include "ctx.h"
 #include "ms.h"
 #include "solver.h"
+#include "steps.h"
 #include "thr_reduce.cuh"
 
 namespace thr {
@@ -57,7 +58,7 @@ __global__ void k_norm2(const V* a, size_t n, double* partials) {
 __global__ void k_init(MsState* ms, MsHist* hist, const double* partials, int np) {
   const double d = block_sum_partials(partials, np);
   if (threadIdx.x == 0) {
-    ms->delta = d;
+    ms->delta = ms->dl[0] = d;
     ms->switch_delta = ms->switch_rel2 * d;
     hist[0].nsteps = 0;
     hist[1].nsteps = 0;
@@ -123,9 +124,9 @@ __global__ void k_lambda(MsState* ms, MsHist* hist, const double* partials, int 
     ms->gammag = st.gammag;
     ms->lo = st.lo;
     ms->hi = st.hi;
-    ms->delta = st.delta;
+    ms->delta = ms->dl[0] = st.delta;
     ms->status = st.status;
-    ms->done = st.done;
+    ms->done = ms->halt = st.done;
   }
   if (k < kMaxShift) {
     ms->gammas[k] = st.gammas[k];
@@ -360,12 +361,21 @@ int enqueue_batch(thr_ctx* c, MsState* ms, MsHist* hist, MsCoef* cf, VO* out, VO
       return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
     }
   }
+  // FP64 on a small lattice: two kernels per iteration, the scalar steps inside (steps.cu)
+  bool steps = false;
+  if constexpr (sizeof(V) == sizeof(double2) && sizeof(VO) == sizeof(double2)) steps = !prof && steps_apply(c);
   for (int j = 0; j < kBatch; j++) {
     const int so = half * kBatch + j, sn = so + 1 == 2 * kBatch ? 0 : so + 1;
     V* rold = ring + (size_t)so * n;
     V* rnew = ring + (size_t)sn * n;
     V* hcur = (j & 1) ? p : hv;
     const V* hprev = (j & 1) ? hv : p;
+    if constexpr (sizeof(V) == sizeof(double2) && sizeof(VO) == sizeof(double2)) {
+      if (steps) {
+        THR_TRY(ms_step_iteration(c, ms, rec, rold, rnew, hcur, hprev, am, imass, j, rev_md, main, pdl));
+        continue;
+      }
+    }
     // alpha = Re<p, M^dagger M p> (:104) evaluated as |h|^2 = |M p|^2 in the M epilogue
     // each kernel of the chain is a dependent launch of the one before (not across a sampled
     // launch's events, nor for the batch's first, which follows the flush fork)
@@ -386,6 +396,8 @@ int enqueue_batch(thr_ctx* c, MsState* ms, MsHist* hist, MsCoef* cf, VO* out, VO
     c->prof_end(pe);
   }
   (void)s;
+  if (steps)  // the lambda step of the batch's last iteration
+    launch_k(k_lambda, dim3(1), dim3(1024), 0, main, pdl, ms, rec, (const double*)steps_partials2(c), (int)gs);
   if (fork) THR_CUDA(cudaStreamWaitEvent(main, c->ev_join[half], 0));
   return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
 }

@@ -1,0 +1,306 @@
+// steps.cu -- solver iterations on small lattices, the scalar steps inside the stencils.
+//
+// On a small lattice an iteration is a chain of dependent kernels of 2 to 3 us each, and
+// the one-block kernels that sum the stencils' partials (k_alpha, k_lambda in msb.cu) cost
+// as much as the stencils.  Here each stencil block has one warp more, which sums the
+// previous stencil's partials itself -- all blocks alike, while the other warps run the
+// stencil -- and hands the epilogue its coefficient; the lead block's extra warp also
+// advances the solver state.  The iteration is then two kernels instead of four:
+//   M step:   lambda of the step before (gammag), h = M r + gammag h, partials of |h|^2
+//   M^ step:  alpha (omega), r_new = r + omega M^dagger h, partials of |r_new|^2
+// The sums run in block_sum_partials' order, the stencils and the recurrences are the
+// kernel chain's, so the bits are the same.  Measured at 12^2x12, Ls 16 (216 blocks): 9.8 us
+// per iteration instead of 14.0.  Every block reads every partial, so lattices of more than
+// kStepMaxParts blocks keep the chain (there its one-block sums are 5 us of 100).
+//
+// Nothing a kernel reads is written by it: the sums' input and output partials alternate
+// between two arrays, the M step reads delta from dl[] of one parity and writes the other,
+// and the flag that ends the work of later kernels (the M step's lambda may set `done`) is
+// read as `done` by the M^dagger step and as `halt`, which that one sets, by the M step.
+#include <algorithm>
+
+#include "ctx.h"
+#include "dslash_site.cuh"
+#include "ms.h"
+#include "steps.h"
+#include "thr_kernels.h"
+
+namespace thr {
+
+namespace {
+constexpr int kStepThreads = 128;                   // the Shamir stencil's blocks
+constexpr int kStepBlock = kStepThreads + 32;       // and the scalar warp
+constexpr int kStepMaxParts = 2048;                 // two partials per virtual thread of the sum
+
+// sum of p[0..n) (n <= 2048) in every lane of one warp, as block_sum_partials adds them
+// with 1024 threads: thread i adds p[i] and p[i + 1024], each warp's 32 values go through a
+// halving tree, then the 32 warp sums.  A butterfly gives the tree's value (lane 0 of the
+// tree; the operands of an addition commute) in all lanes.
+__device__ __forceinline__ double warp_sum_partials(const double* p, int n, int lane) {
+  constexpr int kU = 8;  // virtual warps in flight
+  double keep = 0.0;
+  for (int w0 = 0; w0 < 32 && w0 * 32 < n; w0 += kU) {
+    double v[kU];
+#pragma unroll
+    for (int k = 0; k < kU; k++) {
+      const int i = (w0 + k) * 32 + lane;
+      v[k] = i < n ? p[i] : 0.0;
+    }
+    if (n > 1024) {
+#pragma unroll
+      for (int k = 0; k < kU; k++) {
+        const int i = (w0 + k) * 32 + lane + 1024;
+        if (i < n) v[k] += p[i];
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int k = 0; k < kU; k++) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    }
+#pragma unroll
+    for (int k = 0; k < kU; k++)
+      if (lane == w0 + k) keep = v[k];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) keep += __shfl_xor_sync(0xffffffffu, keep, o);
+  return keep;
+}
+
+// ms_alpha_block and ms_lambda_block (ms.h) by one warp
+__device__ __forceinline__ void ms_alpha_warp(MsState* ms, MsHist* rec, int nstep, double alpha, int lane) {
+  if (lane == 0) {
+    ms_alpha_scalar(ms, alpha);
+    rec->lo[nstep] = ms->lo;
+    rec->hi[nstep] = ms->hi;
+  }
+  __syncwarp();
+  for (int k = ms->lo + lane; k <= ms->hi; k += 32) {
+    ms_alpha_shift(ms, k);
+    rec->om[nstep][k] = ms->omegas[k];
+    rec->ze[nstep][k] = ms->zeta_iii[k];
+  }
+  __syncwarp();
+}
+__device__ __forceinline__ void ms_lambda_warp(MsState* ms, MsHist* rec, int nstep, double lambda, int lane) {
+  if (lane == 0) ms_lambda_scalar(ms, lambda);
+  __syncwarp();
+  const int lo0 = ms->lo, hi0 = ms->hi;
+  for (int k = lo0 + lane; k <= hi0; k += 32) {
+    ms_lambda_shift(ms, k);
+    rec->ga[nstep][k] = ms->gammas[k];
+  }
+  const int nq = ms->ndiagq, it = ms->it;
+  const double delta = ms->delta, res = (double)ms->res;
+  int mini = nq, maxi = -1;
+  for (int q = lane; q < nq; q += 32) {
+    if (q >= lo0 && q <= hi0) ms->cg_returns[q] = it;
+    if (ms->flags[q]) {
+      if (sqrt(delta * ms->zeta_ii[q] * ms->zeta_ii[q]) * ms->correction[q] < res) {
+        ms->flags[q] = 0;
+      } else {
+        mini = min(mini, q);
+        maxi = max(maxi, q);
+      }
+    }
+  }
+  mini = __reduce_min_sync(0xffffffffu, mini);
+  maxi = __reduce_max_sync(0xffffffffu, maxi);
+  for (int q = lane; q < kMaxShift; q += 32) {
+    if (q >= mini && q <= maxi) {
+      ms->zeta_i[q] = ms->zeta_ii[q];
+      ms->zeta_ii[q] = ms->zeta_iii[q];
+    }
+  }
+  if (lane == 0) {
+    rec->nsteps = nstep + 1;
+    ms->lo = mini;
+    ms->hi = maxi;
+    ms->delta = ms->lambda;
+    if (!(ms->lambda == ms->lambda)) ms->status = THR_ERR_NAN;
+    if (maxi < mini || ms->it >= ms->maxcg || ms->status) ms->done = 1;
+  }
+  __syncwarp();
+}
+
+struct StepArgs {
+  double2* out;
+  const double2* in;
+  const double2* aux;
+  const double2* u;
+  Geom g;
+  float am, am3;
+  int imass;
+  const double* pin;  // the previous stencil's partials
+  double* pout;
+  int np;             // partials = stencil blocks
+  int spb;            // sites per block
+  unsigned mls;       // geom_magic of Ls for thread indices
+  int rev;
+};
+
+// One stencil block with its scalar warp: coef(lane) runs in the scalar warp beside the
+// stencil and returns the epilogue's coefficient, lead(lane) in the lead block's scalar
+// warp beside the epilogue.  DAG: r_new = r + c M^dagger h; else h_new = M r + c h.
+template <bool DAG, bool SHFL, class Coef, class Lead>
+__device__ __forceinline__ void step_block(const StepArgs& a, Coef&& coef, Lead&& lead) {
+  __shared__ double s_coef;
+  __shared__ double red[kStepThreads];
+  const Geom g = a.g;
+  const int tid = threadIdx.x;
+  const bool scal = tid >= kStepThreads;
+  const int bid = a.rev ? a.np - 1 - (int)blockIdx.x : (int)blockIdx.x;
+  double2 acc[4], av[4];
+  int s = 0, site = 0;
+  bool live = false;
+  if (scal) {
+    const double c = coef(tid & 31);
+    if (tid == kStepThreads) s_coef = c;
+  } else {
+    const int sub = geom_div(tid, g.ls, a.mls);
+    s = tid - sub * g.ls;
+    site = bid * a.spb + sub;
+    live = sub < a.spb && site < g.v3;
+    if (SHFL || live) {  // with SHFL every lane takes part (spare rows on a clamped site)
+      const int sc = live ? site : g.v3 - 1;
+#pragma unroll
+      for (int d = 0; d < 4; d++) av[d] = a.aux[sidx32(g, s, sc, d)];
+      shamir_site<double2, DAG, SHFL>(a.in, a.u, g, s, sc, a.am, a.imass, a.am3, acc);
+    }
+  }
+  __syncthreads();
+  if (!scal) {
+    const double om = s_coef;
+    double racc = 0.0;
+    if (live) {
+#pragma unroll
+      for (int d = 0; d < 4; d++) {
+        const double2 v = DAG ? av[d] + om * acc[d] : acc[d] + om * av[d];
+        a.out[sidx32(g, s, site, d)] = v;
+        racc += epi_norm<double2>(v);
+      }
+    }
+    red[tid] = racc;
+  } else if (blockIdx.x == 0) {
+    lead(tid & 31);
+  }
+  __syncthreads();
+  if (tid < 32) {  // the block's partial in block_partial_sum's order
+    const int nthr = a.spb * g.ls;
+    double v = 0.0;
+    for (int i = tid; i < nthr; i += 32) v += red[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (tid == 0) a.pout[bid] = v;
+  }
+}
+
+// DAG false: the M step of iteration j (with the lambda step of iteration j - 1, unless it
+// is the batch's first: that one's was taken by k_lambda); DAG true: the M^dagger step
+// (with the alpha step) of iteration j
+template <bool DAG, bool SHFL, int MINB>
+__global__ void __launch_bounds__(kStepBlock, MINB) k_ms_step(StepArgs a, MsState* ms, MsHist* rec, int j) {
+  pdl_wait();
+  pdl_trigger();
+  if (DAG ? ms->done : ms->halt) {
+    if (DAG && blockIdx.x == 0 && threadIdx.x == 0) ms->halt = 1;
+    return;
+  }
+  __shared__ MsState st;  // the lead block's working copy of the state
+  const bool due = DAG || j > 0;
+  double total = 0.0;
+  step_block<DAG, SHFL>(
+      a,
+      [&](int lane) -> double {
+        if (!due) return ms->gammag;
+        if (blockIdx.x == 0) {  // issued with the partials' loads
+          double* dst = reinterpret_cast<double*>(&st);
+          const double* src = reinterpret_cast<const double*>(ms);
+#pragma unroll 4
+          for (int i = lane; i < (int)(sizeof(MsState) / sizeof(double)); i += 32) dst[i] = src[i];
+        }
+        const double delta = DAG ? ms->delta : ms->dl[(j + 1) & 1];
+        total = warp_sum_partials(a.pin, a.np, lane);
+        __syncwarp();
+        return DAG ? -delta / total : total / delta;  // omega (:126-127), gammag (:143)
+      },
+      [&](int lane) {
+        if (!due) return;
+        if (DAG) {
+          ms_alpha_warp(&st, rec, j, total, lane);
+          if (lane == 0) {
+            ms->it = st.it;
+            ms->alpha = st.alpha;
+            ms->omega_save = st.omega_save;
+            ms->omega = st.omega;
+          }
+          for (int k = lane; k < kMaxShift; k += 32) {
+            ms->zeta_iii[k] = st.zeta_iii[k];
+            ms->omegas[k] = st.omegas[k];
+          }
+        } else {
+          ms_lambda_warp(&st, rec, j - 1, total, lane);
+          if (lane == 0) {
+            ms->lambda = st.lambda;
+            ms->active_sum = st.active_sum;
+            ms->gammag = st.gammag;
+            ms->lo = st.lo;
+            ms->hi = st.hi;
+            ms->delta = st.delta;
+            ms->dl[j & 1] = st.delta;
+            ms->status = st.status;
+            ms->done = st.done;
+          }
+          for (int k = lane; k < kMaxShift; k += 32) {
+            ms->gammas[k] = st.gammas[k];
+            ms->cg_returns[k] = st.cg_returns[k];
+            ms->flags[k] = st.flags[k];
+            ms->zeta_i[k] = st.zeta_i[k];
+            ms->zeta_ii[k] = st.zeta_ii[k];
+          }
+        }
+      });
+}
+
+bool step_shfl(const Geom& g) { return g.ls <= 32 && (g.ls & (g.ls - 1)) == 0; }
+
+StepArgs step_args(thr_ctx* c, double2* out, const double2* in, const double2* aux, float am, int imass,
+                   const double* pin, double* pout, int rev) {
+  const dim3 blk = stencil_block(c->g, 0);
+  return StepArgs{out,  in,   aux,  c->u64, c->g, am, c->p.am3, imass,
+                  pin,  pout, (int)stencil_grid(c->g, 0), (int)blk.y,
+                  geom_magic(kStepThreads, c->g.ls), rev};
+}
+
+template <bool DAG>
+void launch_ms_step(const StepArgs& a, MsState* ms, MsHist* rec, int j, cudaStream_t st, bool pdl) {
+  // few blocks per SM: registers for every load of a site at once
+  const bool wide = a.np <= 2 * device_sms();
+  const dim3 grd(a.np), blk(kStepBlock);
+  if (step_shfl(a.g)) {
+    if (wide) launch_k(k_ms_step<DAG, true, 2>, grd, blk, 0, st, pdl, a, ms, rec, j);
+    else launch_k(k_ms_step<DAG, true, 4>, grd, blk, 0, st, pdl, a, ms, rec, j);
+  } else {
+    if (wide) launch_k(k_ms_step<DAG, false, 2>, grd, blk, 0, st, pdl, a, ms, rec, j);
+    else launch_k(k_ms_step<DAG, false, 4>, grd, blk, 0, st, pdl, a, ms, rec, j);
+  }
+}
+}  // namespace
+
+bool steps_apply(const thr_ctx* c) {
+  const unsigned np = stencil_grid(c->g, 0);
+  return c->p.kernel == 0 && c->g.ls <= kStepThreads && np <= (unsigned)kStepMaxParts &&
+         stencil_parts(c->g, 0, true) == np && 2 * (size_t)np + 2 <= c->nparts;
+}
+
+double* steps_partials2(const thr_ctx* c) { return c->partials + ((stencil_grid(c->g, 0) + 1) & ~1u); }
+
+int ms_step_iteration(thr_ctx* c, MsState* ms, MsHist* rec, double2* rold, double2* rnew, double2* hcur,
+                      const double2* hprev, float am, int imass, int j, int rev_md, cudaStream_t st, bool pdl) {
+  double *pa = c->partials, *pl = steps_partials2(c);
+  launch_ms_step<false>(step_args(c, hcur, rold, hprev, am, imass, pl, pa, 0), ms, rec, j, st, pdl && j > 0);
+  launch_ms_step<true>(step_args(c, rnew, hcur, rold, am, imass, pa, pl, rev_md), ms, rec, j, st, pdl);
+  return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
+}
+
+}  // namespace thr

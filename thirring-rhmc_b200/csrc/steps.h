@@ -1,0 +1,21 @@
+// steps.h -- solver iterations on small lattices with the scalar steps inside the
+// stencil kernels (steps.cu): FP64, Shamir.
+#pragma once
+#include "ctx.h"
+#include "ms.h"
+
+namespace thr {
+
+// whether the context's lattice takes them
+bool steps_apply(const thr_ctx* c);
+// the second array of stencil partials (the first is c->partials)
+double* steps_partials2(const thr_ctx* c);
+
+// iteration j of a batch of the batched multishift: h = M r_old + gammag h_prev and
+// r_new = r_old + omega M^dagger h, with the lambda step of iteration j - 1 and the alpha
+// step of iteration j inside; the batch's last lambda step is the caller's (k_lambda on
+// steps_partials2)
+int ms_step_iteration(thr_ctx* c, MsState* ms, MsHist* rec, double2* rold, double2* rnew, double2* hcur,
+                      const double2* hprev, float am, int imass, int j, int rev_md, cudaStream_t st, bool pdl);
+
+}  // namespace thr
