@@ -29,3 +29,22 @@ def test_multishift_steps_bit_identical(dims, layout, maxcg):
     (x, it, cgr), (xc, itc, cgrc) = outs
     assert it == itc and np.array_equal(cgr, cgrc)
     assert np.array_equal(x, xc)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,layout", [((2, 2, 2, 8), 0), ((3, 5, 2, 33), 0), ((4, 6, 10, 20), 1),
+                                         ((12, 12, 12, 16), 0), ((16, 16, 14, 40), 1)])
+def test_congrad_steps_bit_identical(dims, layout):
+    """Congrad's three-kernel iteration against its six-kernel chain: the same bits and counts."""
+    rng = np.random.default_rng(9)
+    L = O.lat(*dims)
+    u, phi = rand_links(L, rng), rand_spinor(L, rng)
+    outs = []
+    with thirring.Lattice(*dims, layout=layout) as G:
+        G.set_links(u)
+        for stride in (0, 1 << 20):
+            G._L.thr_profile(G.h, stride, 1)
+            x = np.zeros_like(phi)
+            outs.append(G.congrad(phi, x, 0.2, 0.05, 3) + (x,))
+    assert outs[0][:2] == outs[1][:2] and outs[0][0] > 2
+    assert np.array_equal(outs[0][2], outs[1][2])

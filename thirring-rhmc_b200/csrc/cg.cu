@@ -10,6 +10,7 @@
 
 #include "ctx.h"
 #include "solver.h"
+#include "steps.h"
 #include "thr_reduce.cuh"
 
 namespace thr {
@@ -119,7 +120,7 @@ __global__ void k_cg_latch(CgState* cs) {
 // whatever the device state holds (congrad itself stops at niterc)
 __global__ void k_cg_loop(CgState* cs, cudaGraphConditionalHandle h) {
   cs->chunks += 1;
-  unsigned more = cs->done ? 0u : 1u;
+  unsigned more = (cs->done || cs->pending_done) ? 0u : 1u;
   if (more && cs->chunks >= cs->max_chunks) {
     cs->status = THR_ERR_MAXITER;
     cs->done = 1;
@@ -146,11 +147,16 @@ int cg_enqueue_chunk(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* r
   // chunk's first, which follows the loop control, excepted; THR_PDL=0: none); each waits
   // for its predecessor before it reads anything, so the results are the same
   const bool pdl = c->use_pdl;
+  const bool steps = !c->prof_on && steps_apply(c);  // the chain while kernels are timed, as the multishift
   for (int k = 0; k < kCgChunk; k++) {
     // sweep directions alternate with the iteration's parity (kCgChunk is even): each
     // kernel starts on the sites its predecessor wrote last (results do not depend on it)
     const int odd = c->rev_sweep == 2 ? (k & 1) : 0;
     const int rev_m = odd, rev_md = c->rev_sweep ? 1 - odd : 0, rev_p = odd;
+    if (steps) {  // small lattices: three kernels, the scalar steps inside (steps.cu)
+      THR_TRY(cg_step_iteration(c, cs, X, p, r, x1, am, imass, k, rev_m, rev_md, rev_p, c->st, pdl));
+      continue;
+    }
     // x1 = M p with alphad = |x1|^2 (:60, :70) from the stencil's epilogue
     THR_TRY(launch_dslash_norm<double2>(c->g, c->p.kernel, false, x1, p, c->u64, am, imass, c->p.am3, c->st,
                                         &cs->done, c->partials, rev_m, pdl && k > 0));
@@ -264,13 +270,13 @@ int congrad_dev(thr_ctx* c, const double2* Phi, double2* X, float res, float am,
   h.resid = (double)resid;
   h.alpha = 1.0;
   h.alphan = 0.0;
-  h.betacgd = 1.0;
+  h.betacgd = h.bd[0] = 1.0;
   h.niterc = niterc;
   h.max_chunks = niterc / kCgChunk + 3;
   THR_CUDA(cudaMemcpyAsync(cs, &h, sizeof(CgState), cudaMemcpyHostToDevice, c->st));
   THR_CUDA(cudaMemcpyAsync(p, X, n * sizeof(double2), cudaMemcpyDeviceToDevice, c->st));
   THR_CUDA(cudaMemcpyAsync(r, Phi, n * sizeof(double2), cudaMemcpyDeviceToDevice, c->st));
-  if (c->use_graphs) {
+  if (c->use_graphs && !c->prof_on) {
     cudaGraphExec_t exec = nullptr;
     THR_TRY(cg_graph(c, cs, X, p, r, x1, x2, am, imass, &exec));
     THR_CUDA(cudaGraphLaunch(exec, c->st));
@@ -281,7 +287,7 @@ int congrad_dev(thr_ctx* c, const double2* Phi, double2* X, float res, float am,
       THR_TRY(cg_enqueue_chunk(c, cs, X, p, r, x1, x2, am, imass));
       THR_CUDA(cudaMemcpyAsync(&h, cs, sizeof(CgState), cudaMemcpyDeviceToHost, c->st));
       THR_CUDA(cudaStreamSynchronize(c->st));
-      if (h.done) break;
+      if (h.done || h.pending_done) break;
     }
   }
   if (itercg) *itercg = h.itercg;

@@ -7,7 +7,10 @@ namespace thr {
 // congrad scalars (measure_module.F90:29-31), kept in device memory
 struct CgState {
   double alpha, alphan, betacg, betacgd, betacgn, resid, nalpha;  // nalpha = -alpha for the fused r update
-  int nx, itercg, niterc, done, pending_done, capped, status, chunks, max_chunks, pad;
+  int nx, itercg, niterc, done, pending_done, capped, status, chunks, max_chunks;
+  // small lattices (steps.cu): |r|^2 before iteration k of a chunk in bd[k & 1] (once started)
+  int started;
+  double bd[2];
 };
 
 template <class S>

@@ -3,6 +3,7 @@
 #pragma once
 #include "ctx.h"
 #include "ms.h"
+#include "solver.h"
 
 namespace thr {
 
@@ -17,5 +18,10 @@ double* steps_partials2(const thr_ctx* c);
 // steps_partials2)
 int ms_step_iteration(thr_ctx* c, MsState* ms, MsHist* rec, double2* rold, double2* rnew, double2* hcur,
                       const double2* hprev, float am, int imass, int j, int rev_md, cudaStream_t st, bool pdl);
+
+// iteration k of a chunk of congrad: h = M p with |h|^2; r -= alpha M^dagger h with |r|^2 and
+// the alpha step inside; x += alpha p, p = r + betacg p with the beta step inside
+int cg_step_iteration(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* r, double2* h, float am, int imass,
+                      int k, int rev_m, int rev_md, int rev_p, cudaStream_t st, bool pdl);
 
 }  // namespace thr
