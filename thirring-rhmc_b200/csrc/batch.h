@@ -31,8 +31,11 @@ struct BatchTable {
   int total_blocks = 0;
   long long total_elems = 0;  // sum of 4*V5 over entries
   long long total_links = 0;  // sum of 3*V3 over distinct link sets
+  int max_blocks = 0;         // work blocks of the largest entry
+  bool even_ls = true;        // every entry's Ls is even
   std::vector<BatchEntry> host;
   BatchEntry* dev = nullptr;
+  int* wmap = nullptr;        // device: the entry of each work block
   ~BatchTable();
   // shared_links: all entries use the links at offset 0 (right-hand sides of one lattice)
   int build(const std::vector<Geom>& geoms, bool shared_links, cudaStream_t st);
@@ -50,5 +53,14 @@ int launch_dslash_batch_fused(const BatchTable& b, int kernel, bool dag, int epi
                               const typename Sto<S>::C* u, float am, int imass, float am3, cudaStream_t st,
                               const int* skip, typename Sto<S>::C* rv, const double* coef, int coef_stride,
                               double* partials, int grid = 0);
+
+struct BcgRun;
+// bstep.cu: one CG step of every entry as three kernels (Shamir; entries of at most
+// kStepMaxBlocks work blocks, whose partials every block of the entry sums); step: the
+// inner solve's step, from 0.  pair_ok: FP32 storage with even Ls
+constexpr int kStepMaxBlocks = 512;
+constexpr int kStepPartials = 8;  // partial slots of a work block, per array
+template <class VS, class VA>
+int launch_bcg_step(BcgRun& br, VA* r, VS* p, VS* h, VA* e, int step, int inner_cap);
 
 }  // namespace thr

@@ -28,7 +28,10 @@
 
 namespace thr {
 
-BatchTable::~BatchTable() { cudaFree(dev); }
+BatchTable::~BatchTable() {
+  cudaFree(dev);
+  cudaFree(wmap);
+}
 
 int BatchTable::build(const std::vector<Geom>& geoms, bool shared_links, cudaStream_t st) {
   host.clear();
@@ -36,6 +39,9 @@ int BatchTable::build(const std::vector<Geom>& geoms, bool shared_links, cudaStr
   total_blocks = 0;
   total_elems = 0;
   total_links = 0;
+  max_blocks = 0;
+  even_ls = true;
+  std::vector<int> map;
   for (const Geom& g : geoms) {
     if (g.ls < 1 || g.ls > 256) return THR_ERR_BADSHAPE;
     BatchEntry e{};
@@ -46,12 +52,20 @@ int BatchTable::build(const std::vector<Geom>& geoms, bool shared_links, cudaStr
     e.nblk = (g.v3 + e.spb - 1) / e.spb;
     e.blk0 = total_blocks;
     total_blocks += e.nblk;
+    max_blocks = std::max(max_blocks, e.nblk);
+    even_ls = even_ls && g.ls % 2 == 0;
+    map.insert(map.end(), (size_t)e.nblk, (int)host.size());
     total_elems += g.v5 * 4;
     if (!shared_links || host.empty()) total_links += (long long)g.v3 * 3;
     host.push_back(e);
   }
   cudaFree(dev);
+  cudaFree(wmap);
   dev = nullptr;
+  wmap = nullptr;
+  if (cudaMalloc(&wmap, sizeof(int) * std::max(1, total_blocks)) != cudaSuccess) return THR_ERR_NOMEM;
+  if (cudaMemcpyAsync(wmap, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice, st) != cudaSuccess)
+    return THR_ERR_CUDA;
   if (cudaMalloc(&dev, sizeof(BatchEntry) * std::max(1, nent)) != cudaSuccess) return THR_ERR_NOMEM;
   if (cudaMemcpyAsync(dev, host.data(), sizeof(BatchEntry) * nent, cudaMemcpyHostToDevice, st) != cudaSuccess)
     return THR_ERR_CUDA;
@@ -170,11 +184,12 @@ __global__ void k_inner_start(BcgState* stt, int* skip, const double* partials, 
   const double rr = warp_entry_sum(partials, e * gx, gx);
   if (threadIdx.x != 0) return;
   BcgState& s = stt[e];
-  s.rr = rr;
+  s.rr = s.rr2[0] = rr;
   s.inner_it = 0;
+  s.iters0 = s.iters;
   s.done_at = -1;  // no step of this inner solve has run
   s.done_inner = s.done_outer || !(rr > s.target);
-  skip[e] = s.done_inner;
+  skip[e] = skip[gridDim.x + e] = s.done_inner;
 }
 
 // pq from the stencil epilogue partials of the entry's work blocks; alpha = rr / pq
@@ -282,6 +297,23 @@ static int bcg_inner(BcgRun& br, VA* r, VS* p, VS* h, VS* q, VA* ev, float tol, 
   k_inner_start<<<tab.nent, 32, 0, br.st>>>(br.state, br.skip, br.partials, kGX);
   const int chunk = 16;
   std::vector<BcgState> h_state(tab.nent);
+  if (br.kernel == 0 && tab.max_blocks <= kStepMaxBlocks) {
+    // three dependent kernels per step; the states of one chunk are looked at while the
+    // next one runs (steps past an entry's end change nothing)
+    constexpr int half = 8;
+    for (int c = 0; half * (c - 2) < inner_cap; c++) {
+      for (int k = 0; k < half; k++) THR_TRY((launch_bcg_step<VS, VA>(br, r, p, h, ev, half * c + k, inner_cap)));
+      br.launches += 3 * half;
+      BcgState* hs = br.hstate + (size_t)(c & 1) * tab.nent;
+      THR_CUDA(cudaMemcpyAsync(hs, br.state, sizeof(BcgState) * tab.nent, cudaMemcpyDeviceToHost, br.st));
+      THR_CUDA(cudaEventRecord(br.ev[c & 1], br.st));
+      if (c == 0) continue;
+      THR_CUDA(cudaEventSynchronize(br.ev[(c - 1) & 1]));
+      hs = br.hstate + (size_t)((c - 1) & 1) * tab.nent;
+      if (std::all_of(hs, hs + tab.nent, [](const BcgState& s) { return s.done_inner != 0; })) break;
+    }
+    return THR_OK;
+  }
   // per step: h = M p with |h|^2 = |M p|^2 (the reference's alphad, :70); alpha; r -= alpha
   // M^dagger h with |r|^2 in the M^dagger epilogue (q = M^dagger M p never stored); beta;
   // e += alpha p and p = r + beta p in one pass.  r is held in the stencil's arithmetic type.

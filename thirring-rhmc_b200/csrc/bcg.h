@@ -10,6 +10,9 @@ struct BcgState {
   double rr, pq, alpha, beta, target, resid, r2_true;
   int iters, inner_it, outer, done_outer, done_inner, cap, status, rounds;
   int done_at;  // inner-loop step whose residual ended the entry's inner solve (-1: none)
+  // three-kernel step (bstep.cu): rr before step k in rr2[k & 1]; iters at the inner solve's start
+  int iters0;
+  double rr2[2];
 };
 
 struct BcgRun {
@@ -22,8 +25,10 @@ struct BcgRun {
   const void* ulow = nullptr;    // links, FP32
   int grid = 0;                  // persistent stencil grid (0 = default)
   BcgState* state = nullptr;     // [nent]
-  int* skip = nullptr;           // [nent]
-  double* partials = nullptr;    // >= max(total_blocks, 64 * nent)
+  int* skip = nullptr;           // [2 nent]: skip, and its copy the x and p update reads
+  double* partials = nullptr;    // >= max(2 kStepPartials total_blocks, 64 * nent)
+  BcgState* hstate = nullptr;    // pinned, 2 x [nent]
+  cudaEvent_t ev[2] = {};        // hstate slots copied
   const double2* B = nullptr;    // right-hand sides, FP64
   double2* X = nullptr;          // solutions, FP64 (initial guesses in)
   double2 *R = nullptr, *T = nullptr, *H = nullptr;  // FP64 work

@@ -29,6 +29,8 @@ struct BatchBufs {
   float2* u32 = nullptr;
   void* stage = nullptr;
   size_t stage_bytes = 0;
+  BcgState* hstate = nullptr;  // pinned
+  cudaEvent_t ev[2] = {};
   ~BatchBufs() { release(); }
   void release() {
     for (void* ptr : {(void*)state, (void*)skip, (void*)partials, (void*)B, (void*)X, (void*)R, (void*)T, (void*)H, r,
@@ -36,12 +38,21 @@ struct BatchBufs {
       cudaFree(ptr);
     state = nullptr; skip = nullptr; partials = nullptr; B = X = R = T = H = nullptr;
     r = p = h = q = e = nullptr; u64 = nullptr; u32 = nullptr; stage = nullptr;
+    if (hstate) cudaFreeHost(hstate);
+    hstate = nullptr;
+    for (cudaEvent_t& v : ev) {
+      if (v) cudaEventDestroy(v);
+      v = nullptr;
+    }
   }
   int alloc(bool own_links, size_t stage_b) {
     const size_t n = (size_t)tab.total_elems, ne = (size_t)tab.nent;
-    const size_t nparts = std::max((size_t)tab.total_blocks, 64 * ne) + 64;
-    bool ok = cudaMalloc(&state, sizeof(BcgState) * ne) == cudaSuccess && cudaMalloc(&skip, sizeof(int) * ne) == cudaSuccess &&
-              cudaMalloc(&partials, sizeof(double) * nparts) == cudaSuccess;
+    const size_t nparts = std::max(2 * kStepPartials * (size_t)tab.total_blocks, 64 * ne) + 64;
+    bool ok = cudaMalloc(&state, sizeof(BcgState) * ne) == cudaSuccess &&
+              cudaMalloc(&skip, sizeof(int) * 2 * ne) == cudaSuccess &&
+              cudaMalloc(&partials, sizeof(double) * nparts) == cudaSuccess &&
+              cudaMallocHost(&hstate, 2 * sizeof(BcgState) * ne) == cudaSuccess;
+    for (cudaEvent_t& v : ev) ok = ok && cudaEventCreateWithFlags(&v, cudaEventDisableTiming) == cudaSuccess;
     for (double2** f : {&B, &X, &R, &T, &H}) ok = ok && cudaMalloc(f, n * sizeof(double2)) == cudaSuccess;
     // the inner vectors are sized for FP64 so any precision fits
     for (void** f : {&r, &p, &h, &q, &e}) ok = ok && cudaMalloc(f, n * sizeof(double2)) == cudaSuccess;
@@ -102,6 +113,9 @@ int run_batch(BatchBufs& bb, cudaStream_t st, int kernel, float am3, const doubl
   br.h = bb.h;
   br.q = bb.q;
   br.e = bb.e;
+  br.hstate = bb.hstate;
+  br.ev[0] = bb.ev[0];
+  br.ev[1] = bb.ev[1];
   const int rc = bcg_solve(br, precision, res, 64, itercg, outer);
   if (launches) *launches += br.launches;
   return rc;

@@ -286,22 +286,6 @@ __global__ void __launch_bounds__(512, 2)
 // for either complex type; for FP64 storage it ran at 45-49 us against the
 // one-s kernel's 38 us on the 32^2x32, Ls 32 lattice, so FP64 keeps one s per
 // thread.)
-__device__ __forceinline__ void ld_pair(const float2* p, unsigned i, float2& a, float2& b) {
-  const float4 v = __ldg(reinterpret_cast<const float4*>(p + i));
-  a = make_float2(v.x, v.y);
-  b = make_float2(v.z, v.w);
-}
-__device__ __forceinline__ void ld_pair(const double2* p, unsigned i, double2& a, double2& b) {
-  a = __ldg(p + i);
-  b = __ldg(p + i + 1);
-}
-__device__ __forceinline__ void st_pair(float2* p, unsigned i, float2 a, float2 b) {
-  *reinterpret_cast<float4*>(p + i) = make_float4(a.x, a.y, b.x, b.y);
-}
-__device__ __forceinline__ void st_pair(double2* p, unsigned i, double2 a, double2 b) {
-  p[i] = a;
-  p[i + 1] = b;
-}
 template <class C, bool DAG, int EPI, int MINB>
 __global__ void __launch_bounds__(64, MINB)
     k_dslash_pair(C* __restrict__ out, const C* __restrict__ in, const C* __restrict__ u, Geom g, float am,
@@ -319,49 +303,8 @@ __global__ void __launch_bounds__(64, MINB)
   double racc = 0.0;
   if (live) {
     const int site = site0;
-    int x, y, t;
-    site_coords(g, site, x, y, t);
-    const Nbr nb = neighbours(g, site, x, y, t);
-    SpinorView<C> Rv{in, g};
-    const int Ls = g.ls;
-    const R diag = (R)((3.0f - am3) + 1.0f);
-    C c0[4], c1[4], a0c[4], a1c[4];
-#pragma unroll
-    for (int d = 0; d < 4; d++) {
-      ld_pair(in, sidx32(g, s0, site, d), c0[d], c1[d]);
-      a0c[d] = diag * c0[d];
-      a1c[d] = diag * c1[d];
-    }
-    const int A = DAG ? 0 : 2, B = DAG ? 2 : 0;  // spins taking R(s+1) / R(s-1)
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      a0c[A + k] = a0c[A + k] - c1[A + k];                                   // s0 + 1 = s1 < Ls
-      if (s0 + 1 < Ls - 1) a1c[A + k] = a1c[A + k] - Rv(s0 + 2, site, A + k);
-      if (s0 > 0) a0c[B + k] = a0c[B + k] - Rv(s0 - 1, site, B + k);
-      a1c[B + k] = a1c[B + k] - c0[B + k];                                   // s1 - 1 = s0
-    }
-    const R a = (R)am;
-    const bool five = imass == 5;
-    const C cA = imass == 1 ? mk(a, R(0)) : mk(R(0), (five && DAG) ? -a : a);
-    const C cB = imass == 1 ? mk(a, R(0)) : mk(R(0), five ? (DAG ? -a : a) : -a);
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      if (s0 + 1 == Ls - 1) a1c[A + k] = a1c[A + k] + cmul(cA, five ? c1[B + k] : Rv(0, site, A + k));
-      if (s0 == 0) a0c[B + k] = a0c[B + k] + cmul(cB, five ? c0[A + k] : Rv(Ls - 1, site, B + k));
-    }
-#pragma unroll
-    for (int mu = 0; mu < 3; mu++) {
-#pragma unroll
-      for (int dir = 0; dir < 2; dir++) {
-        const int ns = dir == 0 ? nb.f[mu] : nb.b[mu];
-        const C W = dir == 0 ? __ldg(u + (size_t)mu * g.v3 + site) : cconj(__ldg(u + (size_t)mu * g.v3 + nb.b[mu]));
-        C r0[4], r1[4];
-#pragma unroll
-        for (int d = 0; d < 4; d++) ld_pair(in, sidx32(g, s0, ns, d), r0[d], r1[d]);
-        hop_projected<C, R>(mu, (dir == 0) != DAG, W, r0, a0c);
-        hop_projected<C, R>(mu, (dir == 0) != DAG, W, r1, a1c);
-      }
-    }
+    C a0c[4], a1c[4];
+    shamir_pair<C, DAG, false>(in, u, g, s0, site, am, imass, am3, a0c, a1c);
 #pragma unroll
     for (int d = 0; d < 4; d++) {
       const unsigned i = sidx32(g, s0, site, d);

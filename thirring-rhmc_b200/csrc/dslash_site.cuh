@@ -175,6 +175,130 @@ __device__ __forceinline__ void shamir_site(const S* __restrict__ in, const type
   }
 }
 
+// The batched solver's stencils (bstep.cu) fix the rounding of diag R(s) - R(s +- 1) to what
+// the compiler makes of it in the one-s batch stencil (k_dslash_batch: the first A spin's
+// product rounded by itself, the others fused), so that solutions and iteration counts do
+// not depend on which of them ran.  diag_minus<ONE>: ONE that rounding, else the
+// compiler's choice; k: the k-th spin of A, 2 + k: of B; acc = diag c.
+template <bool ONE>
+__device__ __forceinline__ float2 diag_minus(int k, float diag, float2 c, float2 acc, float2 n) {
+  if (!ONE) return acc - n;
+  if (k == 0) return make_float2(__fsub_rn(__fmul_rn(diag, c.x), n.x), __fsub_rn(__fmul_rn(diag, c.y), n.y));
+  return make_float2(__fmaf_rn(diag, c.x, -n.x), __fmaf_rn(diag, c.y, -n.y));
+}
+template <bool ONE>
+__device__ __forceinline__ double2 diag_minus(int k, double diag, double2 c, double2 acc, double2 n) {
+  if (!ONE) return acc - n;
+  if (k == 0) return make_double2(__dsub_rn(__dmul_rn(diag, c.x), n.x), __dsub_rn(__dmul_rn(diag, c.y), n.y));
+  return make_double2(__fma_rn(diag, c.x, -n.x), __fma_rn(diag, c.y, -n.y));
+}
+// shamir_site with that rounding
+template <class S, bool DAG>
+__device__ __forceinline__ void shamir_one(const S* __restrict__ in, const typename Sto<S>::C* __restrict__ u,
+                                           const Geom& g, int s, int site, float am, int imass, float am3,
+                                           typename Sto<S>::C* acc) {
+  using R = typename Sto<S>::R;
+  using C = typename Sto<S>::C;
+  int x, y, t;
+  site_coords(g, site, x, y, t);
+  const Nbr nb = neighbours(g, site, x, y, t);
+  SpinorView<S> Rv{in, g};
+  const int Ls = g.ls;
+  const R diag = (R)((3.0f - am3) + 1.0f);
+  const int A = DAG ? 0 : 2, B = DAG ? 2 : 0;  // spins taking R(s+1) / R(s-1)
+  C rc[4];
+#pragma unroll
+  for (int d = 0; d < 4; d++) {
+    rc[d] = Rv(s, site, d);
+    acc[d] = diag * rc[d];
+  }
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    if (s < Ls - 1) acc[A + k] = diag_minus<true>(k, diag, rc[A + k], acc[A + k], Rv(s + 1, site, A + k));
+    if (s > 0) acc[B + k] = diag_minus<true>(2 + k, diag, rc[B + k], acc[B + k], Rv(s - 1, site, B + k));
+  }
+  const R a = (R)am;
+  const bool five = imass == 5;
+  const C cA = imass == 1 ? mk(a, R(0)) : mk(R(0), (five && DAG) ? -a : a);
+  const C cB = imass == 1 ? mk(a, R(0)) : mk(R(0), five ? (DAG ? -a : a) : -a);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    if (s == Ls - 1) acc[A + k] = acc[A + k] + cmul(cA, five ? rc[B + k] : Rv(0, site, A + k));
+    if (s == 0) acc[B + k] = acc[B + k] + cmul(cB, five ? rc[A + k] : Rv(Ls - 1, site, B + k));
+  }
+#pragma unroll
+  for (int mu = 0; mu < 3; mu++) {
+#pragma unroll
+    for (int dir = 0; dir < 2; dir++) {
+      const int ns = dir == 0 ? nb.f[mu] : nb.b[mu];
+      const C W = dir == 0 ? __ldg(u + (size_t)mu * g.v3 + site) : cconj(__ldg(u + (size_t)mu * g.v3 + nb.b[mu]));
+      C r[4];
+#pragma unroll
+      for (int d = 0; d < 4; d++) r[d] = Rv(s, ns, d);
+      hop_projected<C, R>(mu, (dir == 0) != DAG, W, r, acc);
+    }
+  }
+}
+
+// Two consecutive s of one site (s0 even, s0 + 1), Ls even, FP32: the Shamir operator with
+// every spinor access a pair (one 16-byte load instead of two of 8).
+__device__ __forceinline__ void ld_pair(const float2* p, size_t i, float2& a, float2& b) {
+  const float4 v = __ldg(reinterpret_cast<const float4*>(p + i));
+  a = make_float2(v.x, v.y);
+  b = make_float2(v.z, v.w);
+}
+__device__ __forceinline__ void st_pair(float2* p, size_t i, float2 a, float2 b) {
+  *reinterpret_cast<float4*>(p + i) = make_float4(a.x, a.y, b.x, b.y);
+}
+template <class C, bool DAG, bool ONE>
+__device__ __forceinline__ void shamir_pair(const C* __restrict__ in, const C* __restrict__ u, const Geom& g, int s0,
+                                            int site, float am, int imass, float am3, C* a0c, C* a1c) {
+  using R = typename Sto<C>::R;
+  int x, y, t;
+  site_coords(g, site, x, y, t);
+  const Nbr nb = neighbours(g, site, x, y, t);
+  SpinorView<C> Rv{in, g};
+  const int Ls = g.ls;
+  const R diag = (R)((3.0f - am3) + 1.0f);
+  C c0[4], c1[4];
+#pragma unroll
+  for (int d = 0; d < 4; d++) {
+    ld_pair(in, sidx32(g, s0, site, d), c0[d], c1[d]);
+    a0c[d] = diag * c0[d];
+    a1c[d] = diag * c1[d];
+  }
+  const int A = DAG ? 0 : 2, B = DAG ? 2 : 0;  // spins taking R(s+1) / R(s-1)
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    a0c[A + k] = diag_minus<ONE>(k, diag, c0[A + k], a0c[A + k], c1[A + k]);
+    if (s0 + 1 < Ls - 1) a1c[A + k] = diag_minus<ONE>(k, diag, c1[A + k], a1c[A + k], Rv(s0 + 2, site, A + k));
+    if (s0 > 0) a0c[B + k] = diag_minus<ONE>(2 + k, diag, c0[B + k], a0c[B + k], Rv(s0 - 1, site, B + k));
+    a1c[B + k] = diag_minus<ONE>(2 + k, diag, c1[B + k], a1c[B + k], c0[B + k]);
+  }
+  const R a = (R)am;
+  const bool five = imass == 5;
+  const C cA = imass == 1 ? mk(a, R(0)) : mk(R(0), (five && DAG) ? -a : a);
+  const C cB = imass == 1 ? mk(a, R(0)) : mk(R(0), five ? (DAG ? -a : a) : -a);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    if (s0 + 1 == Ls - 1) a1c[A + k] = a1c[A + k] + cmul(cA, five ? c1[B + k] : Rv(0, site, A + k));
+    if (s0 == 0) a0c[B + k] = a0c[B + k] + cmul(cB, five ? c0[A + k] : Rv(Ls - 1, site, B + k));
+  }
+#pragma unroll
+  for (int mu = 0; mu < 3; mu++) {
+#pragma unroll
+    for (int dir = 0; dir < 2; dir++) {
+      const int ns = dir == 0 ? nb.f[mu] : nb.b[mu];
+      const C W = dir == 0 ? __ldg(u + (size_t)mu * g.v3 + site) : cconj(__ldg(u + (size_t)mu * g.v3 + nb.b[mu]));
+      C r0[4], r1[4];
+#pragma unroll
+      for (int d = 0; d < 4; d++) ld_pair(in, sidx32(g, s0, ns, d), r0[d], r1[d]);
+      hop_projected<C, R>(mu, (dir == 0) != DAG, W, r0, a0c);
+      hop_projected<C, R>(mu, (dir == 0) != DAG, W, r1, a1c);
+    }
+  }
+}
+
 // One block's sites of the stencil with its epilogue (blockDim = (Ls, sites per
 // block), NT threads at most; the block's sites are bid * blockDim.y + threadIdx.y).
 // Epilogues (EPI): 0 store out = M in; 2 also one FP64 partial of |out|^2 into
