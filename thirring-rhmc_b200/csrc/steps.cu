@@ -9,8 +9,9 @@
 //   M step:   lambda of the step before (gammag), h = M r + gammag h, partials of |h|^2
 //   M^ step:  alpha (omega), r_new = r + omega M^dagger h, partials of |r_new|^2
 // The sums run in block_sum_partials' order, the stencils and the recurrences are the
-// kernel chain's, so the bits are the same.  Measured at 12^2x12, Ls 16 (216 blocks): 9.8 us
-// per iteration instead of 14.0.  Every block reads every partial, so lattices of more than
+// kernel chain's, so the bits are the same.  Measured at 12^2x12, Ls 16 (216 blocks): 7.8 us
+// per iteration instead of 14.0 (9.8 while the lead block's state copy took a round trip per
+// four rows and every warp waited for the flag first).  Every block reads every partial, so lattices of more than
 // kStepMaxParts blocks keep the chain (there its one-block sums are 5 us of 100).
 //
 // Nothing a kernel reads is written by it: the sums' input and output partials alternate
@@ -21,8 +22,9 @@
 // Congrad's iteration is three kernels instead of six in the same way: M p, the M^dagger
 // step with alpha inside, and the x and p update with beta inside (pending_done, set by the
 // update, is read by the stencils; done, set by the M^dagger step, by the update).  At
-// 12^2x12, Ls 16: 12.6 us per iteration instead of 17.5.
+// 12^2x12, Ls 16: 10.7 us per iteration instead of 17.5.
 #include <algorithm>
+#include <type_traits>
 
 #include "ctx.h"
 #include "dslash_site.cuh"
@@ -146,9 +148,11 @@ struct StepArgs {
 
 // One stencil block with its scalar warp: coef(lane) runs in the scalar warp beside the
 // stencil and returns the epilogue's coefficient, lead(lane) in the lead block's scalar
-// warp beside the epilogue.  DAG: r_new = r + c M^dagger h; else h_new = M r + c h.
-template <bool DAG, bool SHFL, class Coef, class Lead>
-__device__ __forceinline__ void step_block(const StepArgs& a, Coef&& coef, Lead&& lead) {
+// warp beside the epilogue.  EPI 1: r_new = r + c M(^dagger) h; 3: h_new = M r + c h; 2: h =
+// M p (no coefficient, no scalar warp).  stop (this kernel's flag, loaded by every thread)
+// is looked at only before the first store, so that the stencil's loads do not wait for it.
+template <bool DAG, int EPI, bool SHFL, class Coef, class Lead>
+__device__ __forceinline__ bool step_block(const StepArgs& a, const int stop, Coef&& coef, Lead&& lead) {
   __shared__ double s_coef;
   __shared__ double red[kStepThreads];
   const Geom g = a.g;
@@ -168,19 +172,22 @@ __device__ __forceinline__ void step_block(const StepArgs& a, Coef&& coef, Lead&
     live = sub < a.spb && site < g.v3;
     if (SHFL || live) {  // with SHFL every lane takes part (spare rows on a clamped site)
       const int sc = live ? site : g.v3 - 1;
+      if (EPI != 2) {
 #pragma unroll
-      for (int d = 0; d < 4; d++) av[d] = a.aux[sidx32(g, s, sc, d)];
+        for (int d = 0; d < 4; d++) av[d] = a.aux[sidx32(g, s, sc, d)];
+      }
       shamir_site<double2, DAG, SHFL>(a.in, a.u, g, s, sc, a.am, a.imass, a.am3, acc);
     }
   }
-  __syncthreads();
+  if (stop) return false;
+  if (EPI != 2) __syncthreads();
   if (!scal) {
-    const double om = s_coef;
+    const double om = EPI != 2 ? s_coef : 0.0;
     double racc = 0.0;
     if (live) {
 #pragma unroll
       for (int d = 0; d < 4; d++) {
-        const double2 v = DAG ? av[d] + om * acc[d] : acc[d] + om * av[d];
+        const double2 v = EPI == 1 ? av[d] + om * acc[d] : EPI == 3 ? acc[d] + om * av[d] : acc[d];
         a.out[sidx32(g, s, site, d)] = v;
         racc += epi_norm<double2>(v);
       }
@@ -198,6 +205,7 @@ __device__ __forceinline__ void step_block(const StepArgs& a, Coef&& coef, Lead&
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if (tid == 0) a.pout[bid] = v;
   }
+  return true;
 }
 
 // DAG false: the M step of iteration j (with the lambda step of iteration j - 1, unless it
@@ -207,26 +215,30 @@ template <bool DAG, bool SHFL, int MINB>
 __global__ void __launch_bounds__(kStepBlock, MINB) k_ms_step(StepArgs a, MsState* ms, MsHist* rec, int j) {
   pdl_wait();
   pdl_trigger();
-  if (DAG ? ms->done : ms->halt) {
-    if (DAG && blockIdx.x == 0 && threadIdx.x == 0) ms->halt = 1;
-    return;
-  }
   __shared__ MsState st;  // the lead block's working copy of the state
+  constexpr int kWords = (int)(sizeof(MsState) / sizeof(double)), kRows = (kWords + 31) / 32;
   const bool due = DAG || j > 0;
+  const int stop = DAG ? ms->done : ms->halt;
   double total = 0.0;
-  step_block<DAG, SHFL>(
-      a,
+  const bool ran = step_block<DAG, DAG ? 1 : 3, SHFL>(
+      a, stop,
       [&](int lane) -> double {
         if (!due) return ms->gammag;
-        if (blockIdx.x == 0) {  // issued with the partials' loads
-          double* dst = reinterpret_cast<double*>(&st);
-          const double* src = reinterpret_cast<const double*>(ms);
-#pragma unroll 4
-          for (int i = lane; i < (int)(sizeof(MsState) / sizeof(double)); i += 32) dst[i] = src[i];
-        }
         const double delta = DAG ? ms->delta : ms->dl[(j + 1) & 1];
-        total = warp_sum_partials(a.pin, a.np, lane);
-        __syncwarp();
+        if (blockIdx.x == 0) {  // every load of the copy in flight at once
+          const double* src = reinterpret_cast<const double*>(ms);
+          double w[kRows];
+#pragma unroll
+          for (int i = 0; i < kRows; i++) w[i] = lane + 32 * i < kWords ? src[lane + 32 * i] : 0.0;
+          total = warp_sum_partials(a.pin, a.np, lane);
+          double* dst = reinterpret_cast<double*>(&st);
+#pragma unroll
+          for (int i = 0; i < kRows; i++)
+            if (lane + 32 * i < kWords) dst[lane + 32 * i] = w[i];
+          __syncwarp();
+        } else {
+          total = warp_sum_partials(a.pin, a.np, lane);
+        }
         return DAG ? -delta / total : total / delta;  // omega (:126-127), gammag (:143)
       },
       [&](int lane) {
@@ -265,6 +277,7 @@ __global__ void __launch_bounds__(kStepBlock, MINB) k_ms_step(StepArgs a, MsStat
           }
         }
       });
+  if (DAG && !ran && blockIdx.x == 0 && threadIdx.x == 0) ms->halt = 1;
 }
 
 // r -= alpha M^dagger h (measure_module.F90:92) with the alpha step (:57, :66-75) of
@@ -273,13 +286,10 @@ template <bool SHFL, int MINB>
 __global__ void __launch_bounds__(kStepBlock, MINB) k_cg_step(StepArgs a, CgState* cs, int k) {
   pdl_wait();
   pdl_trigger();
-  if (cs->pending_done) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) cs->done = 1;
-    return;
-  }
+  const int stop = cs->pending_done;
   double alpha = 1.0;  // the first iteration's
-  step_block<true, SHFL>(
-      a,
+  const bool ran = step_block<true, 1, SHFL>(
+      a, stop,
       [&](int lane) -> double {
         const int started = cs->started;
         const double rr = cs->bd[k & 1];
@@ -294,6 +304,14 @@ __global__ void __launch_bounds__(kStepBlock, MINB) k_cg_step(StepArgs a, CgStat
           cs->alpha = alpha;
         }
       });
+  if (!ran && blockIdx.x == 0 && threadIdx.x == 0) cs->done = 1;
+}
+// h = M p (:60) with |h|^2 (:70)
+template <bool SHFL, int MINB>
+__global__ void __launch_bounds__(kStepThreads, MINB) k_cg_m_step(StepArgs a, const CgState* cs) {
+  pdl_wait();
+  pdl_trigger();
+  step_block<false, 2, SHFL>(a, cs->pending_done, [](int) { return 0.0; }, [](int) {});
 }
 
 // x = x + alpha*p (:77, skipped at nx == 1), p = r + betacg*p (:119) with the beta step
@@ -303,7 +321,7 @@ __global__ void __launch_bounds__(256) k_cg_update_step(CgState* cs, double2* x,
                                                         unsigned np4, int rev, const double* pin, int np, int k) {
   pdl_wait();
   pdl_trigger();
-  if (cs->done) return;
+  const int stop = cs->done;
   __shared__ double s_rr;
   const double alpha = cs->alpha, rr_old = cs->bd[k & 1];
   const int nx = cs->nx;
@@ -324,6 +342,7 @@ __global__ void __launch_bounds__(256) k_cg_update_step(CgState* cs, double2* x,
     const double v = warp_sum_partials(pin, np, threadIdx.x);
     if (threadIdx.x == 0) s_rr = v;
   }
+  if (stop) return;
   __syncthreads();
   const double rr = s_rr;
   const double beta = nx == 1 ? 0.0 : rr / rr_old;
@@ -397,17 +416,22 @@ int ms_step_iteration(thr_ctx* c, MsState* ms, MsHist* rec, double2* rold, doubl
 int cg_step_iteration(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* r, double2* h, float am, int imass,
                       int k, int rev_m, int rev_md, int rev_p, cudaStream_t st, bool pdl) {
   double *pa = c->partials, *pb = steps_partials2(c);
-  THR_TRY(launch_dslash_norm<double2>(c->g, 0, false, h, p, c->u64, am, imass, c->p.am3, st, &cs->pending_done, pa,
-                                      rev_m, pdl && k > 0));
   const StepArgs a = step_args(c, r, h, r, am, imass, pa, pb, rev_md);
+  const StepArgs m = step_args(c, h, p, nullptr, am, imass, nullptr, pa, rev_m);
   const bool wide = a.np <= 2 * device_sms();
-  const dim3 grd(a.np), blk(kStepBlock);
+  auto run = [&](auto sh, auto mb) {
+    constexpr bool SH = decltype(sh)::value;
+    constexpr int MB = decltype(mb)::value;
+    launch_k(k_cg_m_step<SH, MB>, dim3(a.np), dim3(kStepThreads), 0, st, pdl && k > 0, m, (const CgState*)cs);
+    launch_k(k_cg_step<SH, MB>, dim3(a.np), dim3(kStepBlock), 0, st, pdl, a, cs, k);
+  };
+  using std::integral_constant;
   if (step_shfl(a.g)) {
-    if (wide) launch_k(k_cg_step<true, 2>, grd, blk, 0, st, pdl, a, cs, k);
-    else launch_k(k_cg_step<true, 4>, grd, blk, 0, st, pdl, a, cs, k);
+    if (wide) run(std::true_type{}, integral_constant<int, 2>{});
+    else run(std::true_type{}, integral_constant<int, 4>{});
   } else {
-    if (wide) launch_k(k_cg_step<false, 2>, grd, blk, 0, st, pdl, a, cs, k);
-    else launch_k(k_cg_step<false, 4>, grd, blk, 0, st, pdl, a, cs, k);
+    if (wide) run(std::false_type{}, integral_constant<int, 2>{});
+    else run(std::false_type{}, integral_constant<int, 4>{});
   }
   const unsigned np4 = (unsigned)(c->n4() / 4);
   const unsigned gb = std::min((np4 + 255) / 256, (unsigned)(8 * device_sms()));
