@@ -1340,9 +1340,9 @@ int launch_dslash_norm(const Geom& g, int kernel, bool dag, S* out, const S* in,
 
 template <class S>
 int launch_dslash(const Geom& g, int kernel, bool dag, S* out, const S* in, const typename Sto<S>::C* u, float am,
-                  int imass, float am3, cudaStream_t st, const int* skip) {
-  return launch_dslash_mode<S>(g, kernel, dag, out, in, u, am, imass, am3, st, skip, nullptr, nullptr, nullptr, 0,
-                               0);
+                  int imass, float am3, cudaStream_t st, const int* skip, bool pdl) {
+  return launch_dslash_mode<S>(g, kernel, dag, out, in, u, am, imass, am3, st, skip, nullptr, nullptr, nullptr, 0, 0,
+                               true, pdl);
 }
 
 template <class S>
@@ -1353,12 +1353,12 @@ int launch_dslash_untuned(const Geom& g, int kernel, bool dag, S* out, const S* 
 }
 
 int launch_odslash(const Geom& g, bool dag, double2* out, const double2* in, const double2* u, float am, int imass,
-                   float am3, const double* zc, cudaStream_t st, const int* skip) {
+                   float am3, const double* zc, cudaStream_t st, const int* skip, bool pdl) {
   if (g.ls > 1024) return THR_ERR_BADSHAPE;
   if (4ULL * (unsigned long long)g.v5 >= (1ULL << 32)) return THR_ERR_BADSHAPE;  // 32-bit element offsets
   if (imass != 1 && imass != 3) return THR_ERR_UNSUPPORTED;  // measure_OWilson.F90:66-83
   return launch_wilson<double2, true>(g, dag, out, in, u, am, imass, am3, zc, st, skip, nullptr, nullptr, nullptr, 0, 0,
-                                      true, false);
+                                      true, pdl);
 }
 
 // The persistent batch stencil's grid (resident blocks per SM) is tuned like the register
@@ -1439,7 +1439,7 @@ int launch_dslash_batch_fused(const BatchTable& b, int kernel, bool dag, int epi
 
 #define THR_INST(S, L)                                                                                            \
   template int launch_dslash<S>(const Geom&, int, bool, S*, const S*, const L*, float, int, float, cudaStream_t,   \
-                                const int*);                                                                      \
+                                const int*, bool);                                                                \
   template int launch_dslash_untuned<S>(const Geom&, int, bool, S*, const S*, const L*, float, int, float,        \
                                         cudaStream_t, const int*);                                                \
   template int launch_dslash_axpy<S>(const Geom&, int, bool, S*, const S*, const L*, float, int, float,           \

@@ -465,7 +465,8 @@ int thr_odslash_dev(thr_ctx* c, void* out, const void* in, float am, int imass, 
   cudaSetDevice(c->dev);
   const double* zc = nullptr;
   THR_TRY(zolo_device(c, &zc));
-  return launch_odslash(c->g, dag != 0, (double2*)out, (const double2*)in, c->u64, am, imass, c->p.am3, zc, c->st);
+  return launch_odslash(c->g, dag != 0, (double2*)out, (const double2*)in, c->u64, am, imass, c->p.am3, zc, c->st,
+                        nullptr, c->use_pdl);
 }
 
 int thr_congrad_o(thr_ctx* c, const double* Phi, double* X, float res, int* itercg, float am, int imass,

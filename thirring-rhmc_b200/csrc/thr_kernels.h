@@ -45,7 +45,7 @@ unsigned stencil_parts(const Geom& g, int kernel, bool fp64);
 // dslash.cu
 template <class S>
 int launch_dslash(const Geom& g, int kernel, bool dag, S* out, const S* in, const typename Sto<S>::C* u, float am,
-                  int imass, float am3, cudaStream_t st, const int* skip = nullptr);
+                  int imass, float am3, cudaStream_t st, const int* skip = nullptr, bool pdl = false);
 // as launch_dslash, but never runs the autotuner's timing launches (no events, no
 // synchronisation): the register budget is one tuned earlier in the process or the
 // default, which gives the same results
@@ -67,7 +67,7 @@ int launch_dslash_norm(const Geom& g, int kernel, bool dag, S* out, const S* in,
 
 // odslash / odslashd (measure_OWilson.F90:14-167), FP64, with the slice coefficients zc[0..Ls-1] on the device
 int launch_odslash(const Geom& g, bool dag, double2* out, const double2* in, const double2* u, float am, int imass,
-                   float am3, const double* zc, cudaStream_t st, const int* skip = nullptr);
+                   float am3, const double* zc, cudaStream_t st, const int* skip = nullptr, bool pdl = false);
 
 // hnew = (M or M^dagger) in + (*coef) * hold and one FP64 partial per block of |hnew|^2
 // (hnew and hold distinct fields)
