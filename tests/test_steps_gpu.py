@@ -13,10 +13,12 @@ from helpers import rand_links, rand_spinor
                                          ((12, 12, 12, 16), 0), ((16, 16, 12, 40), 0), ((16, 16, 14, 40), 1),
                                          ((16, 16, 24, 40), 0)])
 @pytest.mark.parametrize("maxcg", [33, 150])
-def test_multishift_steps_bit_identical(dims, layout, maxcg):
+@pytest.mark.parametrize("sp", [False, True])
+def test_multishift_steps_bit_identical(dims, layout, maxcg, sp):
     """One block, idle threads, both site orders, up to 1024 partials and above (two per
     thread of the sum), just under and over the largest lattice that takes the two-kernel
-    iteration; stopped inside a batch: the same bits and counts as the kernel chain."""
+    iteration; stopped inside a batch; FP64 and FP32 vectors (even Ls: two s per thread): the
+    same bits and counts as the kernel chain."""
     rng = np.random.default_rng(5)
     L = O.lat(*dims)
     u, inp = rand_links(L, rng), rand_spinor(L, rng)
@@ -25,7 +27,7 @@ def test_multishift_steps_bit_identical(dims, layout, maxcg):
     with thirring.Lattice(*dims, layout=layout, ndiag=4) as G:
         for stride in (0, 1 << 20):
             G._L.thr_profile(G.h, stride, 1)
-            outs.append(G.multishift_solver(u, 0.05, 3, aden, anum, inp, 1e-7, maxcg))
+            outs.append(G.multishift_solver(u, 0.05, 3, aden, anum, inp, 1e-7, maxcg, sp=sp))
     (x, it, cgr), (xc, itc, cgrc) = outs
     assert it == itc and np.array_equal(cgr, cgrc)
     assert np.array_equal(x, xc)

@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(kBThreads + (DAG ? 32 : 0), MINB) k_bstencil(B
   const S* in = (DAG ? a.h : a.p) + w.off;
   C acc[kPer][4];
   if (live) {
-    if constexpr (PAIR) shamir_pair<C, DAG, true>(in, a.u + w.uoff, g, s, site, a.am, a.imass, a.am3, acc[0], acc[1]);
+    if constexpr (PAIR) shamir_pair<C, DAG>(in, a.u + w.uoff, g, s, site, a.am, a.imass, a.am3, acc[0], acc[1]);
     else shamir_one<S, DAG>(in, a.u + w.uoff, g, s, site, a.am, a.imass, a.am3, acc[0]);
   }
   if constexpr (DAG) {

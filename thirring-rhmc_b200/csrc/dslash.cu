@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(64, MINB)
   if (live) {
     const int site = site0;
     C a0c[4], a1c[4];
-    shamir_pair<C, DAG, false>(in, u, g, s0, site, am, imass, am3, a0c, a1c);
+    shamir_pair<C, DAG>(in, u, g, s0, site, am, imass, am3, a0c, a1c);
 #pragma unroll
     for (int d = 0; d < 4; d++) {
       const unsigned i = sidx32(g, s0, site, d);
@@ -833,7 +833,7 @@ __global__ void __launch_bounds__(256, KER == 0 ? 4 : 2)
       wilson_exchange<S, false, DAG, 256>(in + E.off, u + E.uoff, g, s, site, live, threadIdx.x, am, imass, am3,
                                           nullptr, reinterpret_cast<C*>(wsm), acc);
     } else {
-      if (live) shamir_site<S, DAG, false>(in + E.off, u + E.uoff, g, s, site, am, imass, am3, acc);
+      if (live) shamir_one<S, DAG>(in + E.off, u + E.uoff, g, s, site, am, imass, am3, acc);
     }
     if (live) {
       if (EPI == 4) {

@@ -37,12 +37,11 @@ __device__ __forceinline__ double epi_redot(const S* aux, size_t i, typename Sto
   return (double)t;
 }
 
-// |v|^2 in the working precision, accumulated in FP64
+// |v|^2 in the working precision (x^2 fused onto the rounded y^2), accumulated in FP64
 template <class S>
 __device__ __forceinline__ double epi_norm(typename Sto<S>::C v) {
-  using R = typename Sto<S>::R;
-  const R t = v.x * v.x + v.y * v.y;
-  return (double)t;
+  if constexpr (sizeof(v.x) == sizeof(double)) return __fma_rn(v.x, v.x, __dmul_rn(v.y, v.y));
+  else return (double)__fmaf_rn(v.x, v.x, __fmul_rn(v.y, v.y));
 }
 
 // ---------------------------------------------------------------- Shamir
@@ -91,6 +90,22 @@ __device__ __forceinline__ void hop_projected(int mu, bool plus, C W, const C* r
   }
 }
 
+// The rounding of diag R(s) - R(s +- 1) is fixed, so that solutions and iteration counts do
+// not depend on what the compiler fuses in one kernel or another.  The single-lattice FP64
+// kernels round the product by itself (mul_rn); the batched solver's stencils and the FP32
+// pairs fuse it with the difference for all but the first A spin (diag_minus; k: the k-th
+// spin of A, 2 + k: of B).
+__device__ __forceinline__ double2 mul_rn(double d, double2 a) {
+  return make_double2(__dmul_rn(d, a.x), __dmul_rn(d, a.y));
+}
+__device__ __forceinline__ float2 diag_minus(int k, float diag, float2 c, float2 n) {
+  if (k == 0) return make_float2(__fsub_rn(__fmul_rn(diag, c.x), n.x), __fsub_rn(__fmul_rn(diag, c.y), n.y));
+  return make_float2(__fmaf_rn(diag, c.x, -n.x), __fmaf_rn(diag, c.y, -n.y));
+}
+__device__ __forceinline__ double2 diag_minus(int k, double diag, double2 c, double2 n) {
+  if (k == 0) return make_double2(__dsub_rn(__dmul_rn(diag, c.x), n.x), __dsub_rn(__dmul_rn(diag, c.y), n.y));
+  return make_double2(__fma_rn(diag, c.x, -n.x), __fma_rn(diag, c.y, -n.y));
+}
 // The site-local terms of the Shamir operator (diagonal, fifth-dimension hop, wall mass
 // term) into acc.  SHFL: the fifth-dimension neighbours and wall values come from the
 // lanes of the same site (blockDim.x = Ls a power of two <= 32, so a site's Ls threads
@@ -107,7 +122,8 @@ __device__ __forceinline__ void shamir_local(const S* __restrict__ in, const Geo
 #pragma unroll
   for (int d = 0; d < 4; d++) {
     rc[d] = Rv(s, site, d);
-    acc[d] = diag * rc[d];
+    if constexpr (sizeof(R) == sizeof(double)) acc[d] = mul_rn(diag, rc[d]);
+    else acc[d] = diag * rc[d];
   }
   // fifth-dimension hop (np_third == 1), dirac.F90:80-87 (M), :317-324 (M^dagger):
   // spins A take R(s+1), spins B take R(s-1); A = (2,3) for M, (0,1) for M^dagger
@@ -175,24 +191,7 @@ __device__ __forceinline__ void shamir_site(const S* __restrict__ in, const type
   }
 }
 
-// The batched solver's stencils (bstep.cu) fix the rounding of diag R(s) - R(s +- 1) to what
-// the compiler makes of it in the one-s batch stencil (k_dslash_batch: the first A spin's
-// product rounded by itself, the others fused), so that solutions and iteration counts do
-// not depend on which of them ran.  diag_minus<ONE>: ONE that rounding, else the
-// compiler's choice; k: the k-th spin of A, 2 + k: of B; acc = diag c.
-template <bool ONE>
-__device__ __forceinline__ float2 diag_minus(int k, float diag, float2 c, float2 acc, float2 n) {
-  if (!ONE) return acc - n;
-  if (k == 0) return make_float2(__fsub_rn(__fmul_rn(diag, c.x), n.x), __fsub_rn(__fmul_rn(diag, c.y), n.y));
-  return make_float2(__fmaf_rn(diag, c.x, -n.x), __fmaf_rn(diag, c.y, -n.y));
-}
-template <bool ONE>
-__device__ __forceinline__ double2 diag_minus(int k, double diag, double2 c, double2 acc, double2 n) {
-  if (!ONE) return acc - n;
-  if (k == 0) return make_double2(__dsub_rn(__dmul_rn(diag, c.x), n.x), __dsub_rn(__dmul_rn(diag, c.y), n.y));
-  return make_double2(__fma_rn(diag, c.x, -n.x), __fma_rn(diag, c.y, -n.y));
-}
-// shamir_site with that rounding
+// shamir_site with the batch rounding
 template <class S, bool DAG>
 __device__ __forceinline__ void shamir_one(const S* __restrict__ in, const typename Sto<S>::C* __restrict__ u,
                                            const Geom& g, int s, int site, float am, int imass, float am3,
@@ -214,8 +213,8 @@ __device__ __forceinline__ void shamir_one(const S* __restrict__ in, const typen
   }
 #pragma unroll
   for (int k = 0; k < 2; k++) {
-    if (s < Ls - 1) acc[A + k] = diag_minus<true>(k, diag, rc[A + k], acc[A + k], Rv(s + 1, site, A + k));
-    if (s > 0) acc[B + k] = diag_minus<true>(2 + k, diag, rc[B + k], acc[B + k], Rv(s - 1, site, B + k));
+    if (s < Ls - 1) acc[A + k] = diag_minus(k, diag, rc[A + k], Rv(s + 1, site, A + k));
+    if (s > 0) acc[B + k] = diag_minus(2 + k, diag, rc[B + k], Rv(s - 1, site, B + k));
   }
   const R a = (R)am;
   const bool five = imass == 5;
@@ -250,7 +249,7 @@ __device__ __forceinline__ void ld_pair(const float2* p, size_t i, float2& a, fl
 __device__ __forceinline__ void st_pair(float2* p, size_t i, float2 a, float2 b) {
   *reinterpret_cast<float4*>(p + i) = make_float4(a.x, a.y, b.x, b.y);
 }
-template <class C, bool DAG, bool ONE>
+template <class C, bool DAG>
 __device__ __forceinline__ void shamir_pair(const C* __restrict__ in, const C* __restrict__ u, const Geom& g, int s0,
                                             int site, float am, int imass, float am3, C* a0c, C* a1c) {
   using R = typename Sto<C>::R;
@@ -270,10 +269,10 @@ __device__ __forceinline__ void shamir_pair(const C* __restrict__ in, const C* _
   const int A = DAG ? 0 : 2, B = DAG ? 2 : 0;  // spins taking R(s+1) / R(s-1)
 #pragma unroll
   for (int k = 0; k < 2; k++) {
-    a0c[A + k] = diag_minus<ONE>(k, diag, c0[A + k], a0c[A + k], c1[A + k]);
-    if (s0 + 1 < Ls - 1) a1c[A + k] = diag_minus<ONE>(k, diag, c1[A + k], a1c[A + k], Rv(s0 + 2, site, A + k));
-    if (s0 > 0) a0c[B + k] = diag_minus<ONE>(2 + k, diag, c0[B + k], a0c[B + k], Rv(s0 - 1, site, B + k));
-    a1c[B + k] = diag_minus<ONE>(2 + k, diag, c1[B + k], a1c[B + k], c0[B + k]);
+    a0c[A + k] = diag_minus(k, diag, c0[A + k], c1[A + k]);
+    if (s0 + 1 < Ls - 1) a1c[A + k] = diag_minus(k, diag, c1[A + k], Rv(s0 + 2, site, A + k));
+    if (s0 > 0) a0c[B + k] = diag_minus(2 + k, diag, c0[B + k], Rv(s0 - 1, site, B + k));
+    a1c[B + k] = diag_minus(2 + k, diag, c1[B + k], c0[B + k]);
   }
   const R a = (R)am;
   const bool five = imass == 5;

@@ -361,16 +361,16 @@ int enqueue_batch(thr_ctx* c, MsState* ms, MsHist* hist, MsCoef* cf, VO* out, VO
       return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
     }
   }
-  // FP64 on a small lattice: two kernels per iteration, the scalar steps inside (steps.cu)
-  bool steps = false;
-  if constexpr (sizeof(V) == sizeof(double2) && sizeof(VO) == sizeof(double2)) steps = !prof && steps_apply(c);
+  // small lattices (FP64 and FP32): two kernels per iteration, the scalar steps inside (steps.cu)
+  constexpr bool can_step = sizeof(V) >= sizeof(float2);
+  const bool steps = can_step && !prof && steps_apply(c, fp64);
   for (int j = 0; j < kBatch; j++) {
     const int so = half * kBatch + j, sn = so + 1 == 2 * kBatch ? 0 : so + 1;
     V* rold = ring + (size_t)so * n;
     V* rnew = ring + (size_t)sn * n;
     V* hcur = (j & 1) ? p : hv;
     const V* hprev = (j & 1) ? hv : p;
-    if constexpr (sizeof(V) == sizeof(double2) && sizeof(VO) == sizeof(double2)) {
+    if constexpr (can_step) {
       if (steps) {
         THR_TRY(ms_step_iteration(c, ms, rec, rold, rnew, hcur, hprev, am, imass, j, rev_md, main, pdl));
         continue;

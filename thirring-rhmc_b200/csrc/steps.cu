@@ -130,11 +130,12 @@ __device__ __forceinline__ void ms_lambda_warp(MsState* ms, MsHist* rec, int nst
   __syncwarp();
 }
 
+template <class C>
 struct StepArgs {
-  double2* out;
-  const double2* in;
-  const double2* aux;
-  const double2* u;
+  C* out;
+  const C* in;
+  const C* aux;
+  const C* u;
   Geom g;
   float am, am3;
   int imass;
@@ -151,45 +152,61 @@ struct StepArgs {
 // warp beside the epilogue.  EPI 1: r_new = r + c M(^dagger) h; 3: h_new = M r + c h; 2: h =
 // M p (no coefficient, no scalar warp).  stop (this kernel's flag, loaded by every thread)
 // is looked at only before the first store, so that the stencil's loads do not wait for it.
-template <bool DAG, int EPI, bool SHFL, class Coef, class Lead>
-__device__ __forceinline__ bool step_block(const StepArgs& a, const int stop, Coef&& coef, Lead&& lead) {
+// PER: consecutive s per thread (2: FP32 storage with even Ls, k_dslash_pair's arithmetic).
+template <class C, int PER, bool DAG, int EPI, bool SHFL, class Coef, class Lead>
+__device__ __forceinline__ bool step_block(const StepArgs<C>& a, const int stop, Coef&& coef, Lead&& lead) {
+  using R = typename Sto<C>::R;
+  constexpr int kThr = kStepThreads / PER;
   __shared__ double s_coef;
-  __shared__ double red[kStepThreads];
+  __shared__ double red[kThr];
   const Geom g = a.g;
   const int tid = threadIdx.x;
-  const bool scal = tid >= kStepThreads;
+  const bool scal = tid >= kThr;
   const int bid = a.rev ? a.np - 1 - (int)blockIdx.x : (int)blockIdx.x;
-  double2 acc[4], av[4];
+  C acc[PER][4], av[PER][4];
   int s = 0, site = 0;
   bool live = false;
   if (scal) {
     const double c = coef(tid & 31);
-    if (tid == kStepThreads) s_coef = c;
+    if (tid == kThr) s_coef = c;
   } else {
-    const int sub = geom_div(tid, g.ls, a.mls);
-    s = tid - sub * g.ls;
+    const int row = g.ls / PER, sub = geom_div(tid, row, a.mls);
+    s = PER * (tid - sub * row);
     site = bid * a.spb + sub;
     live = sub < a.spb && site < g.v3;
     if (SHFL || live) {  // with SHFL every lane takes part (spare rows on a clamped site)
       const int sc = live ? site : g.v3 - 1;
       if (EPI != 2) {
 #pragma unroll
-        for (int d = 0; d < 4; d++) av[d] = a.aux[sidx32(g, s, sc, d)];
+        for (int d = 0; d < 4; d++) {
+#pragma unroll
+          for (int k = 0; k < PER; k++) av[k][d] = a.aux[sidx32(g, s, sc, d) + k];
+        }
       }
-      shamir_site<double2, DAG, SHFL>(a.in, a.u, g, s, sc, a.am, a.imass, a.am3, acc);
+      if constexpr (PER == 2) shamir_pair<C, DAG>(a.in, a.u, g, s, sc, a.am, a.imass, a.am3, acc[0], acc[1]);
+      else shamir_site<C, DAG, SHFL>(a.in, a.u, g, s, sc, a.am, a.imass, a.am3, acc[0]);
     }
   }
   if (stop) return false;
   if (EPI != 2) __syncthreads();
   if (!scal) {
-    const double om = EPI != 2 ? s_coef : 0.0;
+    const R om = EPI != 2 ? (R)s_coef : R(0);
     double racc = 0.0;
     if (live) {
 #pragma unroll
       for (int d = 0; d < 4; d++) {
-        const double2 v = EPI == 1 ? av[d] + om * acc[d] : EPI == 3 ? acc[d] + om * av[d] : acc[d];
-        a.out[sidx32(g, s, site, d)] = v;
-        racc += epi_norm<double2>(v);
+        C v[PER];
+#pragma unroll
+        for (int k = 0; k < PER; k++)
+          v[k] = EPI == 1 ? av[k][d] + om * acc[k][d] : EPI == 3 ? acc[k][d] + om * av[k][d] : acc[k][d];
+        const unsigned i = sidx32(g, s, site, d);
+        if constexpr (PER == 2) {
+          st_pair(a.out, i, v[0], v[1]);
+          racc += epi_norm<C>(v[0]) + epi_norm<C>(v[1]);
+        } else {
+          a.out[i] = v[0];
+          racc += epi_norm<C>(v[0]);
+        }
       }
     }
     red[tid] = racc;
@@ -198,7 +215,7 @@ __device__ __forceinline__ bool step_block(const StepArgs& a, const int stop, Co
   }
   __syncthreads();
   if (tid < 32) {  // the block's partial in block_partial_sum's order
-    const int nthr = a.spb * g.ls;
+    const int nthr = a.spb * (g.ls / PER);
     double v = 0.0;
     for (int i = tid; i < nthr; i += 32) v += red[i];
 #pragma unroll
@@ -211,8 +228,9 @@ __device__ __forceinline__ bool step_block(const StepArgs& a, const int stop, Co
 // DAG false: the M step of iteration j (with the lambda step of iteration j - 1, unless it
 // is the batch's first: that one's was taken by k_lambda); DAG true: the M^dagger step
 // (with the alpha step) of iteration j
-template <bool DAG, bool SHFL, int MINB>
-__global__ void __launch_bounds__(kStepBlock, MINB) k_ms_step(StepArgs a, MsState* ms, MsHist* rec, int j) {
+template <class C, int PER, bool DAG, bool SHFL, int MINB>
+__global__ void __launch_bounds__(kStepThreads / PER + 32, MINB)
+    k_ms_step(StepArgs<C> a, MsState* ms, MsHist* rec, int j) {
   pdl_wait();
   pdl_trigger();
   __shared__ MsState st;  // the lead block's working copy of the state
@@ -220,7 +238,7 @@ __global__ void __launch_bounds__(kStepBlock, MINB) k_ms_step(StepArgs a, MsStat
   const bool due = DAG || j > 0;
   const int stop = DAG ? ms->done : ms->halt;
   double total = 0.0;
-  const bool ran = step_block<DAG, DAG ? 1 : 3, SHFL>(
+  const bool ran = step_block<C, PER, DAG, DAG ? 1 : 3, SHFL>(
       a, stop,
       [&](int lane) -> double {
         if (!due) return ms->gammag;
@@ -283,12 +301,12 @@ __global__ void __launch_bounds__(kStepBlock, MINB) k_ms_step(StepArgs a, MsStat
 // r -= alpha M^dagger h (measure_module.F90:92) with the alpha step (:57, :66-75) of
 // iteration k of a chunk
 template <bool SHFL, int MINB>
-__global__ void __launch_bounds__(kStepBlock, MINB) k_cg_step(StepArgs a, CgState* cs, int k) {
+__global__ void __launch_bounds__(kStepBlock, MINB) k_cg_step(StepArgs<double2> a, CgState* cs, int k) {
   pdl_wait();
   pdl_trigger();
   const int stop = cs->pending_done;
   double alpha = 1.0;  // the first iteration's
-  const bool ran = step_block<true, 1, SHFL>(
+  const bool ran = step_block<double2, 1, true, 1, SHFL>(
       a, stop,
       [&](int lane) -> double {
         const int started = cs->started;
@@ -308,10 +326,10 @@ __global__ void __launch_bounds__(kStepBlock, MINB) k_cg_step(StepArgs a, CgStat
 }
 // h = M p (:60) with |h|^2 (:70)
 template <bool SHFL, int MINB>
-__global__ void __launch_bounds__(kStepThreads, MINB) k_cg_m_step(StepArgs a, const CgState* cs) {
+__global__ void __launch_bounds__(kStepThreads, MINB) k_cg_m_step(StepArgs<double2> a, const CgState* cs) {
   pdl_wait();
   pdl_trigger();
-  step_block<false, 2, SHFL>(a, cs->pending_done, [](int) { return 0.0; }, [](int) {});
+  step_block<double2, 1, false, 2, SHFL>(a, cs->pending_done, [](int) { return 0.0; }, [](int) {});
 }
 
 // x = x + alpha*p (:77, skipped at nx == 1), p = r + betacg*p (:119) with the beta step
@@ -374,50 +392,69 @@ __global__ void __launch_bounds__(256) k_cg_update_step(CgState* cs, double2* x,
 
 bool step_shfl(const Geom& g) { return g.ls <= 32 && (g.ls & (g.ls - 1)) == 0; }
 
-StepArgs step_args(thr_ctx* c, double2* out, const double2* in, const double2* aux, float am, int imass,
-                   const double* pin, double* pout, int rev) {
+template <class C>
+StepArgs<C> step_args(thr_ctx* c, C* out, const C* in, const C* aux, float am, int imass, const double* pin,
+                      double* pout, int rev, int per = 1) {
   const dim3 blk = stencil_block(c->g, 0);
-  return StepArgs{out,  in,   aux,  c->u64, c->g, am, c->p.am3, imass,
-                  pin,  pout, (int)stencil_grid(c->g, 0), (int)blk.y,
-                  geom_magic(kStepThreads, c->g.ls), rev};
+  const C* u;
+  if constexpr (sizeof(C) == sizeof(double2)) u = c->u64;
+  else u = c->u32;
+  return StepArgs<C>{out,  in,   aux,  u, c->g, am, c->p.am3, imass,
+                     pin,  pout, (int)stencil_grid(c->g, 0), (int)blk.y,
+                     geom_magic(kStepThreads, c->g.ls / per), rev};
 }
 
-template <bool DAG>
-void launch_ms_step(const StepArgs& a, MsState* ms, MsHist* rec, int j, cudaStream_t st, bool pdl) {
+template <class C, int PER, bool DAG>
+void launch_ms_step(const StepArgs<C>& a, MsState* ms, MsHist* rec, int j, cudaStream_t st, bool pdl) {
   // few blocks per SM: registers for every load of a site at once
   const bool wide = a.np <= 2 * device_sms();
-  const dim3 grd(a.np), blk(kStepBlock);
-  if (step_shfl(a.g)) {
-    if (wide) launch_k(k_ms_step<DAG, true, 2>, grd, blk, 0, st, pdl, a, ms, rec, j);
-    else launch_k(k_ms_step<DAG, true, 4>, grd, blk, 0, st, pdl, a, ms, rec, j);
+  const dim3 grd(a.np), blk(kStepThreads / PER + 32);
+  if (PER == 1 && step_shfl(a.g)) {
+    if (wide) launch_k(k_ms_step<C, PER, DAG, PER == 1, 2>, grd, blk, 0, st, pdl, a, ms, rec, j);
+    else launch_k(k_ms_step<C, PER, DAG, PER == 1, 4>, grd, blk, 0, st, pdl, a, ms, rec, j);
   } else {
-    if (wide) launch_k(k_ms_step<DAG, false, 2>, grd, blk, 0, st, pdl, a, ms, rec, j);
-    else launch_k(k_ms_step<DAG, false, 4>, grd, blk, 0, st, pdl, a, ms, rec, j);
+    if (wide) launch_k(k_ms_step<C, PER, DAG, false, 2>, grd, blk, 0, st, pdl, a, ms, rec, j);
+    else launch_k(k_ms_step<C, PER, DAG, false, 2 + 2 * PER>, grd, blk, 0, st, pdl, a, ms, rec, j);
   }
 }
 }  // namespace
 
-bool steps_apply(const thr_ctx* c) {
+bool steps_apply(const thr_ctx* c, bool fp64) {
   const unsigned np = stencil_grid(c->g, 0);
   return c->p.kernel == 0 && c->g.ls <= kStepThreads && np <= (unsigned)kStepMaxParts &&
-         stencil_parts(c->g, 0, true) == np && 2 * (size_t)np + 2 <= c->nparts;
+         stencil_parts(c->g, 0, fp64) == np && 2 * (size_t)np + 2 <= c->nparts;
 }
 
 double* steps_partials2(const thr_ctx* c) { return c->partials + ((stencil_grid(c->g, 0) + 1) & ~1u); }
 
-int ms_step_iteration(thr_ctx* c, MsState* ms, MsHist* rec, double2* rold, double2* rnew, double2* hcur,
-                      const double2* hprev, float am, int imass, int j, int rev_md, cudaStream_t st, bool pdl) {
+template <class V>
+int ms_step_iteration(thr_ctx* c, MsState* ms, MsHist* rec, V* rold, V* rnew, V* hcur, const V* hprev, float am,
+                      int imass, int j, int rev_md, cudaStream_t st, bool pdl) {
   double *pa = c->partials, *pl = steps_partials2(c);
-  launch_ms_step<false>(step_args(c, hcur, rold, hprev, am, imass, pl, pa, 0), ms, rec, j, st, pdl && j > 0);
-  launch_ms_step<true>(step_args(c, rnew, hcur, rold, am, imass, pa, pl, rev_md), ms, rec, j, st, pdl);
+  auto run = [&](auto per) {
+    constexpr int P = decltype(per)::value;
+    launch_ms_step<V, P, false>(step_args<V>(c, hcur, rold, hprev, am, imass, pl, pa, 0, P), ms, rec, j, st,
+                                pdl && j > 0);
+    launch_ms_step<V, P, true>(step_args<V>(c, rnew, hcur, rold, am, imass, pa, pl, rev_md, P), ms, rec, j, st, pdl);
+  };
+  if constexpr (sizeof(V) == sizeof(float2)) {
+    if (c->g.ls % 2 == 0) run(std::integral_constant<int, 2>{});
+    else run(std::integral_constant<int, 1>{});
+  } else {
+    run(std::integral_constant<int, 1>{});
+  }
   return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
 }
+template int ms_step_iteration<double2>(thr_ctx*, MsState*, MsHist*, double2*, double2*, double2*, const double2*,
+                                        float, int, int, int, cudaStream_t, bool);
+template int ms_step_iteration<float2>(thr_ctx*, MsState*, MsHist*, float2*, float2*, float2*, const float2*, float,
+                                       int, int, int, cudaStream_t, bool);
 
 int cg_step_iteration(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* r, double2* h, float am, int imass,
                       int k, int rev_m, int rev_md, int rev_p, cudaStream_t st, bool pdl) {
   double *pa = c->partials, *pb = steps_partials2(c);
-  const StepArgs a = step_args(c, r, h, r, am, imass, pa, pb, rev_md);
-  const StepArgs m = step_args(c, h, p, nullptr, am, imass, nullptr, pa, rev_m);
+  const StepArgs<double2> a = step_args<double2>(c, r, h, r, am, imass, pa, pb, rev_md);
+  const StepArgs<double2> m = step_args<double2>(c, h, p, nullptr, am, imass, nullptr, pa, rev_m);
   const bool wide = a.np <= 2 * device_sms();
   auto run = [&](auto sh, auto mb) {
     constexpr bool SH = decltype(sh)::value;

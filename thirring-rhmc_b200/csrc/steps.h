@@ -1,5 +1,5 @@
 // steps.h -- solver iterations on small lattices with the scalar steps inside the
-// stencil kernels (steps.cu): FP64, Shamir.
+// stencil kernels (steps.cu): Shamir; the multishift in FP64 and FP32, congrad in FP64.
 #pragma once
 #include "ctx.h"
 #include "ms.h"
@@ -8,7 +8,7 @@
 namespace thr {
 
 // whether the context's lattice takes them
-bool steps_apply(const thr_ctx* c);
+bool steps_apply(const thr_ctx* c, bool fp64 = true);
 // the second array of stencil partials (the first is c->partials)
 double* steps_partials2(const thr_ctx* c);
 
@@ -16,8 +16,9 @@ double* steps_partials2(const thr_ctx* c);
 // r_new = r_old + omega M^dagger h, with the lambda step of iteration j - 1 and the alpha
 // step of iteration j inside; the batch's last lambda step is the caller's (k_lambda on
 // steps_partials2)
-int ms_step_iteration(thr_ctx* c, MsState* ms, MsHist* rec, double2* rold, double2* rnew, double2* hcur,
-                      const double2* hprev, float am, int imass, int j, int rev_md, cudaStream_t st, bool pdl);
+template <class V>
+int ms_step_iteration(thr_ctx* c, MsState* ms, MsHist* rec, V* rold, V* rnew, V* hcur, const V* hprev, float am,
+                      int imass, int j, int rev_md, cudaStream_t st, bool pdl);
 
 // iteration k of a chunk of congrad: h = M p with |h|^2; r -= alpha M^dagger h with |r|^2 and
 // the alpha step inside; x += alpha p, p = r + betacg p with the beta step inside
