@@ -224,9 +224,9 @@ int thr_pack_upload(thr_pack* k, int i, const double* u, const double* Phi, cons
   THR_CUDA(cudaMemcpyAsync(st, u, nl * sizeof(double2), cudaMemcpyHostToDevice, k->st));
   from_fortran_links(g, k->bb.u64 + E.uoff, st, k->st);
   k_links32<<<64, 256, 0, k->st>>>(k->bb.u32 + E.uoff, k->bb.u64 + E.uoff, (size_t)g.v3 * 3);
-  THR_CUDA(cudaMemcpyAsync(st, Phi, nf5_of(g) * sizeof(double2), cudaMemcpyHostToDevice, k->st));
+  THR_TRY(upload_fortran_spinor(g, st, Phi, k->st));
   from_fortran_spinor<double2>(g, k->bb.B + E.off, st, k->st);
-  THR_CUDA(cudaMemcpyAsync(st, X, nf5_of(g) * sizeof(double2), cudaMemcpyHostToDevice, k->st));
+  THR_TRY(upload_fortran_spinor(g, st, X, k->st));
   from_fortran_spinor<double2>(g, k->bb.X + E.off, st, k->st);
   THR_CUDA(cudaStreamSynchronize(k->st));
   return THR_OK;

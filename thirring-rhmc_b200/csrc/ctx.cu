@@ -71,7 +71,7 @@ void thr_ctx::prof_trim(size_t first, long long iters) {
 }
 
 int thr_ctx::upload_spinor(double2* dst, const double* host) {
-  THR_CUDA(cudaMemcpyAsync(stage, host, nf5() * sizeof(double2), cudaMemcpyHostToDevice, st));
+  THR_TRY(upload_fortran_spinor(g, stage, host, st));
   from_fortran_spinor<double2>(g, dst, stage, st);
   return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
 }
@@ -342,7 +342,7 @@ int thr_field_destroy(thr_ctx* c, void* f) {
 int thr_field_upload(thr_ctx* c, void* f, int precision, const double* host) {
   if (!c || !f || !host || !prec_bytes(precision)) return THR_ERR_BADARG;
   cudaSetDevice(c->dev);
-  THR_CUDA(cudaMemcpyAsync(c->stage, host, c->nf5() * sizeof(double2), cudaMemcpyHostToDevice, c->st));
+  THR_TRY(upload_fortran_spinor(c->g, c->stage, host, c->st));
   if (precision == THR_FP64) from_fortran_spinor<double2>(c->g, (double2*)f, c->stage, c->st);
   else if (precision == THR_MIXED_BF16) {
     THR_TRY(c->ensure_w64(1));

@@ -19,34 +19,39 @@ __device__ __forceinline__ size_t f5(const Geom& g, int s, int x, int y, int t, 
          (size_t)(g.ls + 2) * ((size_t)(x + 1) + (size_t)(g.lx + 2) * ((size_t)(y + 1) + (size_t)(g.ly + 2) * ((size_t)(t + 1) + (size_t)(g.lt + 2) * d)));
 }
 
+// The spinor kernels take one row of the fifth dimension per blockDim.x threads: the
+// coordinates are found once per row in 32-bit arithmetic (an element at a time the 64-bit
+// divisions were the kernels' time).
 template <class S>
-__global__ void k_from_fortran_spinor(S* out, const double2* fin, Geom g) {
-  size_t n = (size_t)g.v5 * 4;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    int s = (int)(i % g.ls);
-    size_t r = i / g.ls;
-    int site = (int)(r % g.v3);
-    int d = (int)(r / g.v3);
+__global__ void __launch_bounds__(256) k_from_fortran_spinor(S* out, const double2* fin, Geom g) {
+  const unsigned rows = 4u * (unsigned)g.v3;
+  for (unsigned r = blockIdx.x * blockDim.y + threadIdx.y; r < rows; r += gridDim.x * blockDim.y) {
+    const unsigned d = r / (unsigned)g.v3;
     int x, y, t;
-    site_coords(g, site, x, y, t);
-    double2 v = fin[f5(g, s, x, y, t, d)];
-    Sto<S>::st(out, i, typename Sto<S>::C{(typename Sto<S>::R)v.x, (typename Sto<S>::R)v.y});
+    site_coords(g, (int)(r - d * (unsigned)g.v3), x, y, t);
+    const double2* src = fin + f5(g, 0, x, y, t, (int)d);
+    const size_t dst = (size_t)r * g.ls;
+    for (int s = threadIdx.x; s < g.ls; s += blockDim.x) {
+      const double2 v = src[s];
+      Sto<S>::st(out, dst + s, typename Sto<S>::C{(typename Sto<S>::R)v.x, (typename Sto<S>::R)v.y});
+    }
   }
 }
 
-__global__ void k_to_fortran_spinor(double2* fout, const double2* in, Geom g) {
+__global__ void __launch_bounds__(256) k_to_fortran_spinor(double2* fout, const double2* in, Geom g) {
   // every element of the halo'd array, interior and halos, gets its periodic image
-  const int LS2 = g.ls + 2, LX2 = g.lx + 2, LY2 = g.ly + 2, LT2 = g.lt + 2;
-  size_t n = (size_t)LS2 * LX2 * LY2 * LT2 * 4;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    size_t r = i;
-    int s = (int)(r % LS2); r /= LS2;
-    int x = (int)(r % LX2); r /= LX2;
-    int y = (int)(r % LY2); r /= LY2;
-    int t = (int)(r % LT2);
-    int d = (int)(r / LT2);
-    int ss = wrap(s - 1, g.ls), xx = wrap(x - 1, g.lx), yy = wrap(y - 1, g.ly), tt = wrap(t - 1, g.lt);
-    fout[i] = in[sidx(g, ss, site_index(g, xx, yy, tt), d)];
+  const unsigned LX2 = g.lx + 2, LY2 = g.ly + 2, LT2 = g.lt + 2, rows = 4u * LX2 * LY2 * LT2;
+  const int LS2 = g.ls + 2;
+  for (unsigned i = blockIdx.x * blockDim.y + threadIdx.y; i < rows; i += gridDim.x * blockDim.y) {
+    unsigned r = i / LX2;
+    const int x = wrap((int)(i - r * LX2) - 1, g.lx);
+    const unsigned q = r / LY2;
+    const int y = wrap((int)(r - q * LY2) - 1, g.ly);
+    const unsigned d = q / LT2;
+    const int t = wrap((int)(q - d * LT2) - 1, g.lt);
+    const double2* src = in + sidx(g, 0, site_index(g, x, y, t), (int)d);
+    double2* dst = fout + (size_t)i * LS2;
+    for (int s = threadIdx.x; s < LS2; s += blockDim.x) dst[s] = src[wrap(s - 1, g.ls)];
   }
 }
 
@@ -137,6 +142,15 @@ __global__ void k_to_fortran_ps(float* fout, const float* in, Geom g) {
   }
 }
 
+// threads along a row of n elements, and the grid for `rows` of them in 256-thread blocks
+inline dim3 row_block(int n) {
+  const unsigned tx = n <= 8 ? 8 : n <= 16 ? 16 : 32;
+  return dim3(tx, 256 / tx);
+}
+inline unsigned row_grid(size_t rows, dim3 blk) {
+  const size_t b = (rows + blk.y - 1) / blk.y, most = (size_t)device_sms() * 32;
+  return (unsigned)(b < most ? b : most);
+}
 inline unsigned grid_for(size_t n, int threads = 256) {
   size_t b = (n + threads - 1) / threads;
   if (b > device_sms() * 32) b = device_sms() * 32;
@@ -147,14 +161,33 @@ inline unsigned grid_for(size_t n, int threads = 256) {
 
 template <class S>
 void from_fortran_spinor(const Geom& g, S* out, const double2* fin, cudaStream_t st) {
-  k_from_fortran_spinor<S><<<grid_for((size_t)g.v5 * 4), 256, 0, st>>>(out, fin, g);
+  const dim3 blk = row_block(g.ls);
+  k_from_fortran_spinor<S><<<row_grid((size_t)g.v3 * 4, blk), blk, 0, st>>>(out, fin, g);
 }
 template void from_fortran_spinor<double2>(const Geom&, double2*, const double2*, cudaStream_t);
 template void from_fortran_spinor<float2>(const Geom&, float2*, const double2*, cudaStream_t);
 
 void to_fortran_spinor(const Geom& g, double2* fout, const double2* in, cudaStream_t st) {
-  size_t n = (size_t)(g.ls + 2) * (g.lx + 2) * (g.ly + 2) * (g.lt + 2) * 4;
-  k_to_fortran_spinor<<<grid_for(n), 256, 0, st>>>(fout, in, g);
+  const dim3 blk = row_block(g.ls + 2);
+  k_to_fortran_spinor<<<row_grid((size_t)(g.lx + 2) * (g.ly + 2) * (g.lt + 2) * 4, blk), blk, 0, st>>>(fout, in, g);
+}
+int upload_fortran_spinor(const Geom& g, double2* stage, const double* host, cudaStream_t st) {
+  const size_t plane = (size_t)(g.ls + 2) * (g.lx + 2) * (g.ly + 2) * sizeof(double2);
+  const size_t pitch = plane * (g.lt + 2);
+  cudaError_t e;
+  // page-locked arrays: without the t halos (2 of Lt + 2 planes; a pageable array goes through
+  // the driver's staging buffers faster in one piece: 688 against 720 us at 18x14x10, Ls 20);
+  // 2^31: the largest pitch a 2D copy takes
+  cudaPointerAttributes at;
+  const bool locked = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeHost;
+  if (!locked) cudaGetLastError();
+  if (locked && pitch < (size_t)1 << 31) {
+    e = cudaMemcpy2DAsync(reinterpret_cast<char*>(stage) + plane, pitch, reinterpret_cast<const char*>(host) + plane,
+                          pitch, plane * g.lt, 4, cudaMemcpyHostToDevice, st);
+  } else {
+    e = cudaMemcpyAsync(stage, host, 4 * pitch, cudaMemcpyHostToDevice, st);
+  }
+  return e == cudaSuccess ? THR_OK : THR_ERR_CUDA;
 }
 void to_fortran_noh(const Geom& g, double2* fout, const double2* in, cudaStream_t st) {
   k_to_fortran_noh<<<grid_for((size_t)g.v5 * 4), 256, 0, st>>>(fout, in, g);

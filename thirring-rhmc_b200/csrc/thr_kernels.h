@@ -81,6 +81,9 @@ int launch_dslash_accum(const Geom& g, int kernel, bool dag, S* hnew, const S* i
 template <class S>
 void from_fortran_spinor(const Geom& g, S* out, const double2* fin, cudaStream_t st);
 void to_fortran_spinor(const Geom& g, double2* fout, const double2* in, cudaStream_t st);
+// copies what from_fortran_spinor reads of a host spinor to the same places of `stage`: the
+// t planes inside the halo
+int upload_fortran_spinor(const Geom& g, double2* stage, const double* host, cudaStream_t st);
 // shift outputs (Ls,Lx,Ly,Lt,4) per shift, no halo
 void to_fortran_noh(const Geom& g, double2* fout, const double2* in, cudaStream_t st);
 void from_fortran_noh(const Geom& g, double2* out, const double2* fin, cudaStream_t st);
