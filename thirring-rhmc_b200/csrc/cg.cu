@@ -219,7 +219,7 @@ int cg_graph_build(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* r, 
   THR_TRY(launch_dslash_norm<double2>(c->g, c->p.kernel, false, x1, p, c->u64, am, imass, c->p.am3, c->st, &cs->done,
                                       c->partials));
   THR_TRY(launch_dslash_axpy<double2>(c->g, c->p.kernel, true, x2, x1, c->u64, am, imass, c->p.am3, c->st, &cs->done,
-                                      x2, &cs->nalpha, c->partials, c->rev_sweep ? 1 : 0));
+                                      r, &cs->nalpha, c->partials, c->rev_sweep ? 1 : 0));
   THR_CUDA(cudaGraphCreate(&G.graph, 0));
   cudaGraphConditionalHandle handle;
   THR_CUDA(cudaGraphConditionalHandleCreate(&handle, G.graph, 1, cudaGraphCondAssignDefault));

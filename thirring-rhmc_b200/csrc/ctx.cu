@@ -374,15 +374,15 @@ int thr_dslash_dev(thr_ctx* c, void* out, const void* in, int precision, float a
   switch (precision) {
     case THR_FP64:
       return launch_dslash<double2>(c->g, c->p.kernel, dag != 0, (double2*)out, (const double2*)in, c->u64, am, imass,
-                                    c->p.am3, c->st, nullptr, c->use_pdl);
+                                    c->p.am3, c->st, nullptr, c->dependent_launch());
     case THR_FP32_REF:
     case THR_MIXED_FP32:
       return launch_dslash<float2>(c->g, c->p.kernel, dag != 0, (float2*)out, (const float2*)in, c->u32, am, imass,
-                                   c->p.am3, c->st, nullptr, c->use_pdl);
+                                   c->p.am3, c->st, nullptr, c->dependent_launch());
     case THR_MIXED_BF16:
       return launch_dslash<__nv_bfloat162>(c->g, c->p.kernel, dag != 0, (__nv_bfloat162*)out,
                                            (const __nv_bfloat162*)in, c->u32, am, imass, c->p.am3, c->st, nullptr,
-                                           c->use_pdl);
+                                           c->dependent_launch());
     default: return THR_ERR_BADARG;
   }
 }

@@ -169,4 +169,10 @@ struct thr_ctx {
   int use_links(const double* u_host);                    // NULL keeps current links
   int coef_dev(const float* theta_dev);                   // gauge.F90 coef on device theta
   int sync();
+  // whether a call enqueued now may launch as a programmatic dependent of the kernel before it
+  // (not into a stream capture of the caller's)
+  bool dependent_launch() const {
+    cudaStreamCaptureStatus cs;
+    return use_pdl && cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+  }
 };

@@ -1091,6 +1091,7 @@ int launch_wilson(const Geom& g, bool dag, S* out, const S* in, const typename S
 #undef THR_WE
 #undef THR_W
   int minb = kTuneWilson[0];
+  may_tune = may_tune && aux != out;  // an update in place cannot be repeated for timing
   if (storage_id<S>() < 2 && nt == 128) {
     const TuneKey key{dev, storage_id<S>(), OV ? 2 : 1, dag ? 1 : 0, e, g.lx, g.ly, g.lt, g.ls, g.layout};
     minb = may_tune ? tune_pick(key, kTuneWilson, 3, st, launch) : tune_lookup(key, kTuneWilson);
@@ -1301,6 +1302,7 @@ int launch_dslash_mode(const Geom& g, int kernel, bool dag, S* out, const S* in,
   }
   const int* cand = split_ok ? cand64 : kTuneShamir;
   int minb = cand[0];
+  may_tune = may_tune && aux != out;  // an update in place cannot be repeated for timing
   if (tunable) {
     int dev = 0;
     cudaGetDevice(&dev);

@@ -466,7 +466,7 @@ int thr_odslash_dev(thr_ctx* c, void* out, const void* in, float am, int imass, 
   const double* zc = nullptr;
   THR_TRY(zolo_device(c, &zc));
   return launch_odslash(c->g, dag != 0, (double2*)out, (const double2*)in, c->u64, am, imass, c->p.am3, zc, c->st,
-                        nullptr, c->use_pdl);
+                        nullptr, c->dependent_launch());
 }
 
 int thr_congrad_o(thr_ctx* c, const double* Phi, double* X, float res, int* itercg, float am, int imass,
