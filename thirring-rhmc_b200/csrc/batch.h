@@ -59,7 +59,6 @@ struct BcgRun;
 // kStepMaxBlocks work blocks, whose partials every block of the entry sums); step: the
 // inner solve's step, from 0.  pair_ok: FP32 storage with even Ls
 constexpr int kStepMaxBlocks = 512;
-constexpr int kStepPartials = 8;  // partial slots of a work block, per array
 template <class VS, class VA>
 int launch_bcg_step(BcgRun& br, VA* r, VS* p, VS* h, VA* e, int step, int inner_cap);
 

@@ -26,7 +26,7 @@ struct BcgRun {
   int grid = 0;                  // persistent stencil grid (0 = default)
   BcgState* state = nullptr;     // [nent]
   int* skip = nullptr;           // [2 nent]: skip, and its copy the x and p update reads
-  double* partials = nullptr;    // >= max(2 kStepPartials total_blocks, 64 * nent)
+  double* partials = nullptr;    // >= max(2 total_blocks, 64 * nent)
   BcgState* hstate = nullptr;    // pinned, 2 x [nent]
   cudaEvent_t ev[2] = {};        // hstate slots copied
   const double2* B = nullptr;    // right-hand sides, FP64

@@ -47,7 +47,7 @@ struct BatchBufs {
   }
   int alloc(bool own_links, size_t stage_b) {
     const size_t n = (size_t)tab.total_elems, ne = (size_t)tab.nent;
-    const size_t nparts = std::max(2 * kStepPartials * (size_t)tab.total_blocks, 64 * ne) + 64;
+    const size_t nparts = std::max(2 * (size_t)tab.total_blocks, 64 * ne) + 64;
     bool ok = cudaMalloc(&state, sizeof(BcgState) * ne) == cudaSuccess &&
               cudaMalloc(&skip, sizeof(int) * 2 * ne) == cudaSuccess &&
               cudaMalloc(&partials, sizeof(double) * nparts) == cudaSuccess &&

@@ -11,7 +11,7 @@
 // constant during the solve) before it waits.
 //
 // Measured against the five kernels (one B200): six FP64 lattices of 8^3x8 to 14^3x20 in a
-// pack 33 us per iteration instead of 48; eight FP32 right-hand sides on 16^3, Ls 24 66
+// pack 27 us per iteration instead of 48; eight FP32 right-hand sides on 16^3, Ls 24 66
 // instead of 112 (there the pair accesses of even Ls count most).  Entries of more than
 // kStepMaxBlocks work blocks keep the five: every block of an entry reads all its partials.
 //
@@ -20,10 +20,11 @@
 // kernel (read by the stencils) and copied to skip2 by the M^dagger kernel (read by the
 // last).
 //
-// The partials are one per warp: the stencils' blocks are smaller than a work block of 256
-// threads (finer tail), and the consumer adds a work block's warps in block_partial's order
-// and the work blocks in warp_entry_sum's, so FP64 sums keep the bits of the five-kernel step.
-// (FP32 pairs: a block is a work block and writes one partial.)
+// A stencil block is a work block and writes one partial, summed in block_partial's order, and
+// the consumer adds an entry's partials in warp_entry_sum's, so FP64 sums keep the bits of the
+// five-kernel step.  (Half work blocks with a partial per warp had a finer tail, but every
+// block of the next kernel then reads eight times as many partials: 33 instead of 27 us per
+// iteration for the pack below.)
 #include "batch.h"
 #include "bcg.h"
 #include "dslash_site.cuh"
@@ -32,8 +33,8 @@
 namespace thr {
 
 namespace {
-constexpr int kBThreads = 128;  // stencil threads of a block
-constexpr int kWPart = kStepPartials;
+// stencil threads of a block: a work block, one s per thread (PAIR: two)
+constexpr int b_threads(bool pair) { return pair ? 128 : 256; }
 
 // loads of fields the kernel also writes (not through the read-only path)
 __device__ __forceinline__ void ldw_pair(const float2* p, size_t i, float2& a, float2& b) {
@@ -66,39 +67,19 @@ __device__ __forceinline__ Work work_of(const BatchEntry* tab, const int* wmap, 
   return w;
 }
 
-// sum of the entry's partials in every lane of a warp, NW per work block; the loads of four
-// rounds of work blocks are in flight together
-template <int NW>
+// sum of the entry's partials (one per work block) in every lane of a warp, in
+// warp_entry_sum's order; eight loads in flight
 __device__ __forceinline__ double entry_sum(const double* part, int blk0, int nblk, int lane) {
-  constexpr int kU = 4;
-  part += (size_t)blk0 * NW;
+  constexpr int kU = 8;
+  part += blk0;
   double v = 0.0;
   for (int i0 = lane; i0 < nblk; i0 += 32 * kU) {
-    double w[kU][NW];
+    double w[kU];
 #pragma unroll
-    for (int r = 0; r < kU; r++) {
-      const int i = i0 + 32 * r;
-      if constexpr (NW == 1) {
-        w[r][0] = i < nblk ? __ldcg(part + i) : 0.0;
-      } else {
+    for (int r = 0; r < kU; r++) w[r] = i0 + 32 * r < nblk ? __ldcg(part + i0 + 32 * r) : 0.0;
 #pragma unroll
-        for (int k = 0; k < NW / 2; k++) {
-          const double2 t = i < nblk ? __ldcg(reinterpret_cast<const double2*>(part + (size_t)i * NW) + k) : mk(0.0, 0.0);
-          w[r][2 * k] = t.x;
-          w[r][2 * k + 1] = t.y;
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < kU; r++) {
-#pragma unroll
-      for (int o = NW / 2; o > 0; o >>= 1) {
-#pragma unroll
-        for (int k = 0; k < NW; k++)
-          if (k < o) w[r][k] += w[r][k + o];
-      }
-      if (i0 + 32 * r < nblk) v += w[r][0];
-    }
+    for (int r = 0; r < kU; r++)
+      if (i0 + 32 * r < nblk) v += w[r];
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -122,24 +103,24 @@ struct BStep {
 
 // The stencils.  DAG false: h = M p, partials of |h|^2.  DAG true: r -= alpha M^dagger h,
 // alpha = rr / |h|^2, partials of |r|^2, with a warp more for alpha.  PAIR: two consecutive s
-// per thread (FP32, even Ls: 16-byte accesses), a block per work block; else one s per
-// thread, two blocks per work block.
+// per thread (FP32, even Ls: 16-byte accesses), else one s per thread.  A block per work
+// block.
 template <class S, bool DAG, bool PAIR, int MINB>
-__global__ void __launch_bounds__(kBThreads + (DAG ? 32 : 0), MINB) k_bstencil(BStep<S> a) {
+__global__ void __launch_bounds__(b_threads(PAIR) + (DAG ? 32 : 0), MINB) k_bstencil(BStep<S> a) {
   using C = typename Sto<S>::C;
   using R = typename Sto<S>::R;
   __shared__ R s_alpha;
-  constexpr int kSplit = PAIR ? 1 : 2, kPer = PAIR ? 2 : 1;
+  constexpr int kPer = PAIR ? 2 : 1, kThr = b_threads(PAIR);
   const int tid = threadIdx.x, lane = tid & 31;
-  const int wb = (int)blockIdx.x / kSplit, half = (int)blockIdx.x % kSplit;
+  const int wb = blockIdx.x;
   const Work w = work_of(a.tab, a.wmap, wb);
   const Geom g = w.g;
-  const int vt = half * kBThreads + tid, row = g.ls / kPer;
-  const int sub = vt / row, s = kPer * (vt - sub * row);
+  const int row = g.ls / kPer;
+  const int sub = tid / row, s = kPer * (tid - sub * row);
   const int site = (wb - w.blk0) * w.spb + sub;
-  const bool scal = DAG && tid >= kBThreads;
+  const bool scal = DAG && tid >= kThr;
   const bool live = !scal && sub < w.spb && site < g.v3;
-  const bool lead = wb == w.blk0 && half == 0;
+  const bool lead = wb == w.blk0;
   pdl_wait();
   pdl_trigger();
   if (a.skip[w.e]) {
@@ -155,7 +136,7 @@ __global__ void __launch_bounds__(kBThreads + (DAG ? 32 : 0), MINB) k_bstencil(B
   if constexpr (DAG) {
     if (scal) {
       const double rr = a.stt[w.e].rr2[a.step & 1];
-      const double alpha = rr / entry_sum<PAIR ? 1 : kWPart>(a.pa, w.blk0, w.nblk, lane);
+      const double alpha = rr / entry_sum(a.pa, w.blk0, w.nblk, lane);
       if (lane == 0) {
         s_alpha = (R)alpha;
         if (lead) a.stt[w.e].alpha = alpha;
@@ -198,13 +179,12 @@ __global__ void __launch_bounds__(kBThreads + (DAG ? 32 : 0), MINB) k_bstencil(B
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) racc += __shfl_down_sync(0xffffffffu, racc, o);
   double* part = DAG ? a.pb : a.pa;
-  if constexpr (PAIR) {  // a whole work block: one partial
-    __shared__ double red[kBThreads / 32];
-    if (lane == 0) red[tid >> 5] = racc;
-    asm volatile("bar.sync 1, %0;" ::"n"(kBThreads) : "memory");  // the stencil's threads only
-    if (tid == 0) part[wb] = (red[0] + red[1]) + (red[2] + red[3]);
-  } else {
-    if (lane == 0) part[(size_t)wb * kWPart + half * (kBThreads / 32) + (tid >> 5)] = racc;
+  __shared__ double red[kThr / 32];
+  if (lane == 0) red[tid >> 5] = racc;
+  asm volatile("bar.sync 1, %0;" ::"n"(kThr) : "memory");  // the stencil's threads only
+  if (tid == 0) {  // in block_partial's order
+    if constexpr (PAIR) part[wb] = (red[0] + red[1]) + (red[2] + red[3]);
+    else part[wb] = ((red[0] + red[4]) + (red[2] + red[6])) + ((red[1] + red[5]) + (red[3] + red[7]));
   }
 }
 
@@ -212,7 +192,7 @@ __global__ void __launch_bounds__(kBThreads + (DAG ? 32 : 0), MINB) k_bstencil(B
 // advances its state and raises skip when its solve has ended.  A block per work block,
 // each thread the four spins of one s (PAIR: two).
 template <class S, bool PAIR>
-__global__ void __launch_bounds__(PAIR ? 128 : 256, PAIR ? 6 : 2) k_bxp(BStep<S> a) {
+__global__ void __launch_bounds__(b_threads(PAIR), PAIR ? 6 : 3) k_bxp(BStep<S> a) {
   using C = typename Sto<S>::C;
   using R = typename Sto<S>::R;
   __shared__ double s_rn;
@@ -249,7 +229,7 @@ __global__ void __launch_bounds__(PAIR ? 128 : 256, PAIR ? 6 : 2) k_bxp(BStep<S>
     }
   }
   if (tid < 32) {
-    const double rn = entry_sum<PAIR ? 1 : kWPart>(a.pb, w.blk0, w.nblk, tid);
+    const double rn = entry_sum(a.pb, w.blk0, w.nblk, tid);
     if (tid == 0) s_rn = rn;
   }
   __syncthreads();
@@ -296,10 +276,10 @@ __global__ void __launch_bounds__(PAIR ? 128 : 256, PAIR ? 6 : 2) k_bxp(BStep<S>
 // MB, MD: resident blocks per SM of the M and the (larger) M^dagger blocks
 template <class S, bool PAIR, int MB, int MD>
 void launch_step(const BStep<S>& a, int blocks, cudaStream_t st) {
-  constexpr int kSplit = PAIR ? 1 : 2;
-  launch_k(k_bstencil<S, false, PAIR, MB>, dim3(kSplit * blocks), dim3(kBThreads), 0, st, true, a);
-  launch_k(k_bstencil<S, true, PAIR, MD>, dim3(kSplit * blocks), dim3(kBThreads + 32), 0, st, true, a);
-  launch_k(k_bxp<S, PAIR>, dim3(blocks), dim3(PAIR ? 128 : 256), 0, st, true, a);
+  constexpr int kThr = b_threads(PAIR);
+  launch_k(k_bstencil<S, false, PAIR, MB>, dim3(blocks), dim3(kThr), 0, st, true, a);
+  launch_k(k_bstencil<S, true, PAIR, MD>, dim3(blocks), dim3(kThr + 32), 0, st, true, a);
+  launch_k(k_bxp<S, PAIR>, dim3(blocks), dim3(kThr), 0, st, true, a);
 }
 }  // namespace
 
@@ -319,7 +299,7 @@ int launch_bcg_step(BcgRun& br, VA* r, VS* p, VS* h, VA* e, int step, int inner_
   a.r = reinterpret_cast<C*>(r);
   a.e = reinterpret_cast<C*>(e);
   a.pa = br.partials;
-  a.pb = br.partials + (size_t)kWPart * t.total_blocks;
+  a.pb = br.partials + t.total_blocks;
   a.am = br.am;
   a.am3 = br.am3;
   a.imass = br.imass;
@@ -328,10 +308,10 @@ int launch_bcg_step(BcgRun& br, VA* r, VS* p, VS* h, VA* e, int step, int inner_
   // FP64: with few blocks per SM, registers for a site's loads at once
   if constexpr (sizeof(VS) == sizeof(float2)) {
     if (t.even_ls) launch_step<VS, true, 8, 6>(a, t.total_blocks, br.st);
-    else launch_step<VS, false, 6, 5>(a, t.total_blocks, br.st);
+    else launch_step<VS, false, 3, 3>(a, t.total_blocks, br.st);
   } else {
-    if (2 * t.total_blocks <= 4 * device_sms()) launch_step<VS, false, 3, 3>(a, t.total_blocks, br.st);
-    else launch_step<VS, false, 6, 5>(a, t.total_blocks, br.st);
+    if (t.total_blocks <= device_sms()) launch_step<VS, false, 1, 1>(a, t.total_blocks, br.st);
+    else launch_step<VS, false, 3, 3>(a, t.total_blocks, br.st);
   }
   return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
 }
