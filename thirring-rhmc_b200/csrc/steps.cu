@@ -4,15 +4,17 @@
 // the one-block kernels that sum the stencils' partials (k_alpha, k_lambda in msb.cu) cost
 // as much as the stencils.  Here each stencil block has one warp more, which sums the
 // previous stencil's partials itself -- all blocks alike, while the other warps run the
-// stencil -- and hands the epilogue its coefficient; the lead block's extra warp also
-// advances the solver state.  The iteration is then two kernels instead of four:
+// stencil -- and hands the epilogue its coefficient; a lead block beyond the stencil's has
+// only that warp at work and advances the solver state.  The iteration is then two kernels
+// instead of four:
 //   M step:   lambda of the step before (gammag), h = M r + gammag h, partials of |h|^2
 //   M^ step:  alpha (omega), r_new = r + omega M^dagger h, partials of |r_new|^2
 // The sums run in block_sum_partials' order, the stencils and the recurrences are the
-// kernel chain's, so the bits are the same.  Measured at 12^2x12, Ls 16 (216 blocks): 7.8 us
-// per iteration instead of 14.0 (9.8 while the lead block's state copy took a round trip per
-// four rows and every warp waited for the flag first).  Every block reads every partial, so lattices of more than
-// kStepMaxParts blocks keep the chain (there its one-block sums are 5 us of 100).
+// kernel chain's, so the bits are the same.  Measured at 12^2x12, Ls 16 (216 blocks): 7.5 us
+// per iteration instead of 14.0 (7.9 with the state advanced by a stencil block, 9.8 while
+// its copy took a round trip per four rows and every warp waited for the flag first).  Every
+// block reads every partial, so lattices of more than kStepMaxParts blocks keep the chain
+// (there its one-block sums are 5 us of 100).
 //
 // Nothing a kernel reads is written by it: the sums' input and output partials alternate
 // between two arrays, the M step reads delta from dl[] of one parity and writes the other,
@@ -148,8 +150,8 @@ struct StepArgs {
 };
 
 // One stencil block with its scalar warp: coef(lane) runs in the scalar warp beside the
-// stencil and returns the epilogue's coefficient, lead(lane) in the lead block's scalar
-// warp beside the epilogue.  EPI 1: r_new = r + c M(^dagger) h; 3: h_new = M r + c h; 2: h =
+// stencil and returns the epilogue's coefficient, lead(lane) after it in the lead block
+// (the grid's last, which has no sites).  EPI 1: r_new = r + c M(^dagger) h; 3: h_new = M r + c h; 2: h =
 // M p (no coefficient, no scalar warp).  stop (this kernel's flag, loaded by every thread)
 // is looked at only before the first store, so that the stencil's loads do not wait for it.
 // PER: consecutive s per thread (2: FP32 storage with even Ls, k_dslash_pair's arithmetic).
@@ -162,6 +164,7 @@ __device__ __forceinline__ bool step_block(const StepArgs<C>& a, const int stop,
   const Geom g = a.g;
   const int tid = threadIdx.x;
   const bool scal = tid >= kThr;
+  const bool leadb = EPI != 2 && blockIdx.x == gridDim.x - 1;  // the block beyond the stencil's
   const int bid = a.rev ? a.np - 1 - (int)blockIdx.x : (int)blockIdx.x;
   C acc[PER][4], av[PER][4];
   int s = 0, site = 0;
@@ -169,7 +172,8 @@ __device__ __forceinline__ bool step_block(const StepArgs<C>& a, const int stop,
   if (scal) {
     const double c = coef(tid & 31);
     if (tid == kThr) s_coef = c;
-  } else {
+    if (leadb && !stop) lead(tid & 31);
+  } else if (!leadb) {
     const int row = g.ls / PER, sub = geom_div(tid, row, a.mls);
     s = PER * (tid - sub * row);
     site = bid * a.spb + sub;
@@ -188,6 +192,7 @@ __device__ __forceinline__ bool step_block(const StepArgs<C>& a, const int stop,
     }
   }
   if (stop) return false;
+  if (leadb) return true;
   if (EPI != 2) __syncthreads();
   if (!scal) {
     const R om = EPI != 2 ? (R)s_coef : R(0);
@@ -210,8 +215,6 @@ __device__ __forceinline__ bool step_block(const StepArgs<C>& a, const int stop,
       }
     }
     red[tid] = racc;
-  } else if (blockIdx.x == 0) {
-    lead(tid & 31);
   }
   __syncthreads();
   if (tid < 32) {  // the block's partial in block_partial_sum's order
@@ -243,7 +246,7 @@ __global__ void __launch_bounds__(kStepThreads / PER + 32, MINB)
       [&](int lane) -> double {
         if (!due) return ms->gammag;
         const double delta = DAG ? ms->delta : ms->dl[(j + 1) & 1];
-        if (blockIdx.x == 0) {  // every load of the copy in flight at once
+        if (blockIdx.x == gridDim.x - 1) {  // every load of the copy in flight at once
           const double* src = reinterpret_cast<const double*>(ms);
           double w[kRows];
 #pragma unroll
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(kStepThreads / PER + 32, MINB)
           }
         }
       });
-  if (DAG && !ran && blockIdx.x == 0 && threadIdx.x == 0) ms->halt = 1;
+  if (DAG && !ran && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) ms->halt = 1;
 }
 
 // r -= alpha M^dagger h (measure_module.F90:92) with the alpha step (:57, :66-75) of
@@ -322,7 +325,7 @@ __global__ void __launch_bounds__(kStepBlock, MINB) k_cg_step(StepArgs<double2> 
           cs->alpha = alpha;
         }
       });
-  if (!ran && blockIdx.x == 0 && threadIdx.x == 0) cs->done = 1;
+  if (!ran && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) cs->done = 1;
 }
 // h = M p (:60) with |h|^2 (:70)
 template <bool SHFL, int MINB>
@@ -408,7 +411,7 @@ template <class C, int PER, bool DAG>
 void launch_ms_step(const StepArgs<C>& a, MsState* ms, MsHist* rec, int j, cudaStream_t st, bool pdl) {
   // few blocks per SM: registers for every load of a site at once
   const bool wide = a.np <= 2 * device_sms();
-  const dim3 grd(a.np), blk(kStepThreads / PER + 32);
+  const dim3 grd(a.np + 1), blk(kStepThreads / PER + 32);
   if (PER == 1 && step_shfl(a.g)) {
     if (wide) launch_k(k_ms_step<C, PER, DAG, PER == 1, 2>, grd, blk, 0, st, pdl, a, ms, rec, j);
     else launch_k(k_ms_step<C, PER, DAG, PER == 1, 4>, grd, blk, 0, st, pdl, a, ms, rec, j);
@@ -460,7 +463,7 @@ int cg_step_iteration(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* 
     constexpr bool SH = decltype(sh)::value;
     constexpr int MB = decltype(mb)::value;
     launch_k(k_cg_m_step<SH, MB>, dim3(a.np), dim3(kStepThreads), 0, st, pdl && k > 0, m, (const CgState*)cs);
-    launch_k(k_cg_step<SH, MB>, dim3(a.np), dim3(kStepBlock), 0, st, pdl, a, cs, k);
+    launch_k(k_cg_step<SH, MB>, dim3(a.np + 1), dim3(kStepBlock), 0, st, pdl, a, cs, k);
   };
   using std::integral_constant;
   if (step_shfl(a.g)) {
