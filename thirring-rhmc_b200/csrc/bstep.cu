@@ -11,7 +11,7 @@
 // constant during the solve) before it waits.
 //
 // Measured against the five kernels (one B200): six FP64 lattices of 8^3x8 to 14^3x20 in a
-// pack 27 us per iteration instead of 48; eight FP32 right-hand sides on 16^3, Ls 24 66
+// pack 28 us per iteration instead of 48; eight FP32 right-hand sides on 16^3, Ls 24 66
 // instead of 112 (there the pair accesses of even Ls count most).  Entries of more than
 // kStepMaxBlocks work blocks keep the five: every block of an entry reads all its partials.
 //
@@ -23,7 +23,7 @@
 // A stencil block is a work block and writes one partial, summed in block_partial's order, and
 // the consumer adds an entry's partials in warp_entry_sum's, so FP64 sums keep the bits of the
 // five-kernel step.  (Half work blocks with a partial per warp had a finer tail, but every
-// block of the next kernel then reads eight times as many partials: 33 instead of 27 us per
+// block of the next kernel then reads eight times as many partials: 33 instead of 28 us per
 // iteration for the pack below.)
 #include "batch.h"
 #include "bcg.h"
