@@ -407,17 +407,48 @@ StepArgs<C> step_args(thr_ctx* c, C* out, const C* in, const C* aux, float am, i
                      geom_magic(kStepThreads, c->g.ls / per), rev};
 }
 
+constexpr int kStepMaxShflBudget = 4;
+
+// launch(integral_constant<int, MB>): the resident blocks per SM that a kernel's registers are
+// budgeted for.  One wave of blocks with as many registers as that leaves (a site's loads in
+// flight at once); a grid of more than six blocks per SM runs in several waves anyway, and
+// four keep its loads together.  FP64 multishift, us per iteration with budgets 2 to 6 (the
+// rule's marked): 343 blocks (14^3, Ls 16) 12.6 [8.5] 10.4 12.1 14.8; 549 (14^3, Ls 24) 15.9 16.4
+// [12.2] 13.3 15.5; 683 (16^3, Ls 20) 20.8 17.2 18.6 [15.2] 16.4; 820 (16^3, Ls 24) 23.5 19.5 20.3
+// 22.5 [18.1]; 1000 (20^3, Ls 16) 29.0 25.5 [22.1] 25.0 31.7.  Congrad's stencils alike (343: 13.8
+// [12.9] 14.3 15.2 17.4; 683: 24.0 22.4 23.3 [19.7] 21.1).
+// Up to four blocks s -+ 1 comes by shuffles where Ls allows it (343 blocks: 8.5 against 9.4);
+// in the registers that five or six leave they spill, and the neighbours are read (729 blocks,
+// 18^3, Ls 16: 15.3 against 16.9; 800, 20^2 x 16, Ls 16: 18.2 against 24.0).
+template <class F>
+void with_budget(int blocks, F&& launch) {
+  using std::integral_constant;
+  const int sms = device_sms();
+  if (blocks <= 2 * sms) launch(integral_constant<int, 2>{});
+  else if (blocks <= 3 * sms) launch(integral_constant<int, 3>{});
+  else if (blocks <= 4 * sms || blocks > 6 * sms) launch(integral_constant<int, 4>{});
+  else if (blocks <= 5 * sms) launch(integral_constant<int, 5>{});
+  else launch(integral_constant<int, 6>{});
+}
+
 template <class C, int PER, bool DAG>
 void launch_ms_step(const StepArgs<C>& a, MsState* ms, MsHist* rec, int j, cudaStream_t st, bool pdl) {
-  // few blocks per SM: registers for every load of a site at once
-  const bool wide = a.np <= 2 * device_sms();
   const dim3 grd(a.np + 1), blk(kStepThreads / PER + 32);
-  if (PER == 1 && step_shfl(a.g)) {
-    if (wide) launch_k(k_ms_step<C, PER, DAG, PER == 1, 2>, grd, blk, 0, st, pdl, a, ms, rec, j);
-    else launch_k(k_ms_step<C, PER, DAG, PER == 1, 4>, grd, blk, 0, st, pdl, a, ms, rec, j);
-  } else {
-    if (wide) launch_k(k_ms_step<C, PER, DAG, false, 2>, grd, blk, 0, st, pdl, a, ms, rec, j);
-    else launch_k(k_ms_step<C, PER, DAG, false, 2 + 2 * PER>, grd, blk, 0, st, pdl, a, ms, rec, j);
+  auto go = [&](auto mb) {
+    constexpr int MB = decltype(mb)::value;
+    if constexpr (PER == 1 && MB <= kStepMaxShflBudget) {
+      if (step_shfl(a.g)) {
+        launch_k(k_ms_step<C, PER, DAG, true, MB>, grd, blk, 0, st, pdl, a, ms, rec, j);
+        return;
+      }
+    }
+    launch_k(k_ms_step<C, PER, DAG, false, MB>, grd, blk, 0, st, pdl, a, ms, rec, j);
+  };
+  if constexpr (PER == 1) {
+    with_budget(a.np, go);
+  } else {  // blocks of 96 threads: six of them leave the registers a site needs
+    if (a.np <= 2 * device_sms()) go(std::integral_constant<int, 2>{});
+    else go(std::integral_constant<int, 6>{});
   }
 }
 }  // namespace
@@ -458,21 +489,21 @@ int cg_step_iteration(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* 
   double *pa = c->partials, *pb = steps_partials2(c);
   const StepArgs<double2> a = step_args<double2>(c, r, h, r, am, imass, pa, pb, rev_md);
   const StepArgs<double2> m = step_args<double2>(c, h, p, nullptr, am, imass, nullptr, pa, rev_m);
-  const bool wide = a.np <= 2 * device_sms();
-  auto run = [&](auto sh, auto mb) {
-    constexpr bool SH = decltype(sh)::value;
+  with_budget(a.np, [&](auto mb) {
     constexpr int MB = decltype(mb)::value;
-    launch_k(k_cg_m_step<SH, MB>, dim3(a.np), dim3(kStepThreads), 0, st, pdl && k > 0, m, (const CgState*)cs);
-    launch_k(k_cg_step<SH, MB>, dim3(a.np + 1), dim3(kStepBlock), 0, st, pdl, a, cs, k);
-  };
-  using std::integral_constant;
-  if (step_shfl(a.g)) {
-    if (wide) run(std::true_type{}, integral_constant<int, 2>{});
-    else run(std::true_type{}, integral_constant<int, 4>{});
-  } else {
-    if (wide) run(std::false_type{}, integral_constant<int, 2>{});
-    else run(std::false_type{}, integral_constant<int, 4>{});
-  }
+    auto run = [&](auto sh) {
+      constexpr bool SH = decltype(sh)::value;
+      launch_k(k_cg_m_step<SH, MB>, dim3(a.np), dim3(kStepThreads), 0, st, pdl && k > 0, m, (const CgState*)cs);
+      launch_k(k_cg_step<SH, MB>, dim3(a.np + 1), dim3(kStepBlock), 0, st, pdl, a, cs, k);
+    };
+    if constexpr (MB <= kStepMaxShflBudget) {
+      if (step_shfl(a.g)) {
+        run(std::true_type{});
+        return;
+      }
+    }
+    run(std::false_type{});
+  });
   const unsigned np4 = (unsigned)(c->n4() / 4);
   const unsigned gb = std::min((np4 + 255) / 256, (unsigned)(8 * device_sms()));
   launch_k(k_cg_update_step, dim3(gb), dim3(256), 0, st, pdl, cs, X, p, (const double2*)r, np4, rev_p,
