@@ -40,3 +40,27 @@ def test_step_against_five_kernels(shapes, precision):
     else:
         assert np.max(np.abs(its - its5)) <= 2
         assert all(np.linalg.norm(x - y) <= 1e-6 * np.linalg.norm(y) for x, y in zip(xs, xs5))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shapes", [[(12, 12, 12, 16), (10, 10, 10, 12)], [(12, 12, 12, 16)] * 4,
+                                    [(16, 16, 16, 16), (16, 16, 12, 16)]])
+def test_step_register_budgets(shapes):
+    """156, 432 and 448 work blocks (two and three per SM of 148 cost no wave more than four; four),
+    FP64: the five-kernel step's bits and counts."""
+    rng = np.random.default_rng(8)
+    data = []
+    for dims in shapes + [LARGE]:
+        L = O.lat(*dims)
+        data.append((rand_links(L, rng, beta=2.0), rand_spinor(L, rng)))
+    outs = []
+    for n in (len(shapes), len(shapes) + 1):
+        pack = thirring.Pack((shapes + [LARGE])[:n])
+        for i in range(n):
+            pack.upload(i, data[i][0], data[i][1], np.zeros_like(data[i][1]))
+        its, _ = pack.congrad(1e-3, 0.2, 1, thirring.FP64)
+        outs.append((its[:len(shapes)], [interior(pack.download(i)) for i in range(len(shapes))]))
+        pack.close()
+    (its, xs), (its5, xs5) = outs
+    assert np.array_equal(its, its5)
+    assert all(np.array_equal(x, y) for x, y in zip(xs, xs5))

@@ -305,13 +305,19 @@ int launch_bcg_step(BcgRun& br, VA* r, VS* p, VS* h, VA* e, int step, int inner_
   a.imass = br.imass;
   a.step = step;
   a.cap = inner_cap;
-  // FP64: with few blocks per SM, registers for a site's loads at once
   if constexpr (sizeof(VS) == sizeof(float2)) {
     if (t.even_ls) launch_step<VS, true, 8, 6>(a, t.total_blocks, br.st);
     else launch_step<VS, false, 3, 3>(a, t.total_blocks, br.st);
   } else {
-    if (t.total_blocks <= device_sms()) launch_step<VS, false, 1, 1>(a, t.total_blocks, br.st);
-    else launch_step<VS, false, 3, 3>(a, t.total_blocks, br.st);
+    // as many registers as do not cost a wave of blocks against four per SM.  FP64, us per
+    // iteration with 2 / 3 / 4 per SM: 156 blocks 16.7 / 17.9 / 16.8; 432 - / 20.3 / 22.4; 512 - /
+    // 28.5 / 25.1; 648 - / 30.6 / 31.4; 1145 - / 46.9 / 43.1; 1832 89 / 79 / 76.5
+    const int sms = device_sms();
+    auto waves = [&](int per) { return (t.total_blocks + per * sms - 1) / (per * sms); };
+    if (t.total_blocks <= sms) launch_step<VS, false, 1, 1>(a, t.total_blocks, br.st);
+    else if (waves(2) == waves(4)) launch_step<VS, false, 2, 2>(a, t.total_blocks, br.st);
+    else if (waves(3) == waves(4)) launch_step<VS, false, 3, 3>(a, t.total_blocks, br.st);
+    else launch_step<VS, false, 4, 4>(a, t.total_blocks, br.st);
   }
   return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
 }
