@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(kChainThreads, 512 / kChainThreads) k_ms_chain
     if (gave_up) {
       if (tid == 0) {
         m->status = THR_ERR_TIMEOUT;
-        m->done = 1;
+        m->done = m->halt = 1;
       }
     } else {
       // the fields an iteration changes (not batches or flush_fields: the side stream's
@@ -255,14 +255,14 @@ __global__ void __launch_bounds__(kChainThreads, 512 / kChainThreads) k_ms_chain
       if (tid == 0) {
         m->omega = st.omega;
         m->gammag = st.gammag;
-        m->delta = st.delta;
+        m->delta = m->dl[0] = st.delta;  // dl, halt: the low-precision phase may run in steps.cu's kernels
         m->alpha = st.alpha;
         m->lambda = st.lambda;
         m->omega_save = st.omega_save;
         m->it = st.it;
         m->lo = st.lo;
         m->hi = st.hi;
-        m->done = st.done;
+        m->done = m->halt = st.done;
         m->status = st.status;
         m->active_sum = st.active_sum;
       }
