@@ -992,11 +992,12 @@ bool capturing(cudaStream_t st) {
 template <class S> constexpr int storage_id() { return sizeof(S) == sizeof(double2) ? 0 : sizeof(S) == sizeof(float2) ? 1 : 2; }
 }  // namespace
 
-// the tuned candidate for `key`: looked up, forced by THR_TUNE=<n>, or timed now
-// (each candidate 1 + 3 launches on the call's own fields) unless the stream is
-// being captured; cand[0] when tuning is off or cannot run
+// the tuned candidate for `key`: looked up, forced by THR_TUNE=<n> (and then recorded, so
+// that the report shows it), or timed now (each candidate 1 + 3 launches on the call's own
+// fields) unless the stream is being captured or may_time is false (an update in place,
+// which cannot be repeated); cand[0] when tuning is off or cannot run
 template <class F>
-int tune_pick(const TuneKey& key, const int* cand, int ncand, cudaStream_t st, F&& launch) {
+int tune_pick(const TuneKey& key, const int* cand, int ncand, cudaStream_t st, F&& launch, bool may_time = true) {
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tune.find(key);
@@ -1004,11 +1005,15 @@ int tune_pick(const TuneKey& key, const int* cand, int ncand, cudaStream_t st, F
   }
   if (!tune_on()) return cand[0];
   if (g_tune_force) {
-    for (int c = 0; c < ncand; c++)
-      if (cand[c] == g_tune_force) return g_tune_force;
+    for (int c = 0; c < ncand; c++) {
+      if (cand[c] != g_tune_force) continue;
+      std::lock_guard<std::mutex> lock(g_tune_mu);
+      g_tune[key] = TuneVal{g_tune_force, 0, {}};
+      return g_tune_force;
+    }
     return cand[0];
   }
-  if (capturing(st)) return cand[0];
+  if (!may_time || capturing(st)) return cand[0];
   TuneVal tv{cand[0], ncand, {}};
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess) return cand[0];
@@ -1091,10 +1096,9 @@ int launch_wilson(const Geom& g, bool dag, S* out, const S* in, const typename S
 #undef THR_WE
 #undef THR_W
   int minb = kTuneWilson[0];
-  may_tune = may_tune && aux != out;  // an update in place cannot be repeated for timing
   if (storage_id<S>() < 2 && nt == 128) {
     const TuneKey key{dev, storage_id<S>(), OV ? 2 : 1, dag ? 1 : 0, e, g.lx, g.ly, g.lt, g.ls, g.layout};
-    minb = may_tune ? tune_pick(key, kTuneWilson, 3, st, launch) : tune_lookup(key, kTuneWilson);
+    minb = may_tune ? tune_pick(key, kTuneWilson, 3, st, launch, aux != out) : tune_lookup(key, kTuneWilson);
   }
   launch(minb);
   return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
@@ -1302,12 +1306,11 @@ int launch_dslash_mode(const Geom& g, int kernel, bool dag, S* out, const S* in,
   }
   const int* cand = split_ok ? cand64 : kTuneShamir;
   int minb = cand[0];
-  may_tune = may_tune && aux != out;  // an update in place cannot be repeated for timing
   if (tunable) {
     int dev = 0;
     cudaGetDevice(&dev);
     const TuneKey key{dev, storage_id<S>(), kernel, dag ? 1 : 0, e, g.lx, g.ly, g.lt, g.ls, g.layout};
-    minb = may_tune ? tune_pick(key, cand, ncand, st, launch) : tune_lookup(key, cand);
+    minb = may_tune ? tune_pick(key, cand, ncand, st, launch, aux != out) : tune_lookup(key, cand);
   }
   launch(minb);
 #undef THR_D
