@@ -1,4 +1,5 @@
-"""The stencil tuner: candidates forced by THR_TUNE=<n>, and the report's account of them."""
+"""The stencil tuner's candidates: forced by THR_TUNE=<n>, each gives the default's bits in
+every epilogue, and the report names the candidate that ran."""
 import os
 import subprocess
 import sys
@@ -32,6 +33,45 @@ def _inputs(tmp_path, dims, kernel):
         np.save(tmp_path / (k + ".npy"), v)
 
 
+CASES = [(1, n, ls) for n in (4, 8) for ls in (5, 12, 32, 48, 100)]
+CASES += [(0, n, ls) for n, ls in ((7, 16), (6, 12), (40, 16), (224, 16), (223, 48), (242, 32), (281, 48), (108, 16),
+                                   (106, 32))]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel,force,ls", CASES)
+def test_forced_candidate_same_bits(tmp_path, kernel, force, ls):
+    """M and M^dagger of the Shamir, Wilson and (Wilson's candidates) overlap kernels, the
+    fused epilogues with |out|^2, and congrad in the kernel chain (which runs while kernels
+    are timed), whose M^dagger updates r in place.  150 sites: the last site group of every
+    block shape is part empty and the two-, four- and eight-group blocks have a tail."""
+    dims = (5, 6, 5, ls)
+    _inputs(tmp_path, dims, kernel)
+    ov = kernel == 1 and ls <= 32  # the overlap coefficients are defined to Ls 32
+    body = ("with thirring.Lattice(*%r, kernel=%d) as G:\n"
+            "    G.set_links(u); G._L.thr_profile(G.h, 1 << 20, 1)\n"
+            "    X = np.zeros_like(R); r['it'] = G.congrad(R, X, 0.2, 0.05, 3)[0]; r['x'] = X\n"
+            "    r['m'], r['md'] = G.dslash(R, None, 0.05, 3), G.dslashd(R, None, 0.05, 1)\n"
+            "    for e in (0, 1, 3):\n"
+            "        for dag in (0, 1):\n"
+            "            k = '%%d%%d' %% (e, dag)\n"
+            "            r['f' + k], r['n' + k] = G.dslash_fused(R, A, 0.3, 0.05, 3, dag, e)\n"
+            "    if %r:\n"
+            "        r['o'], r['od'] = G.odslash(R, None, 0.05, 3), G.odslashd(R, None, 0.05, 1)\n" % (dims, kernel, ov))
+    ref = _run(tmp_path, "ref", body, {"THR_TUNE": "0"})
+    got = _run(tmp_path, "alt", body, {"THR_TUNE": str(force)})
+    assert int(ref["it"]) > 2
+    for k in ref.files:
+        if k != "rep":
+            assert np.array_equal(ref[k], got[k]), k
+    ops = [("wilson" if kernel else "shamir", e) for e in (0, 1, 2, 3)] + ([("overlap", 0)] if ov else [])
+    rep = str(got["rep"])
+    for op, e in ops:
+        for d in ("M", "Mdag"):
+            line = "fp64 %s %s epi=%d 5x6x5 Ls=%d layout=0 dev=0 minb=%d " % (op, d, e, ls, force)
+            assert line in rep, (line, rep)
+
+
 @pytest.mark.gpu
 def test_forced_candidate_reaches_updates_in_place(tmp_path):
     """Congrad's M^dagger in the kernel chain writes r over itself: never timed, but a forced
@@ -44,3 +84,16 @@ def test_forced_candidate_reaches_updates_in_place(tmp_path):
     got = _run(tmp_path, "alt", body, {"THR_TUNE": "7"})
     assert int(ref["it"]) == int(got["it"]) and np.array_equal(ref["x"], got["x"])
     assert "fp64 shamir Mdag epi=1 8x6x4 Ls=16 layout=0 dev=0 minb=7 " in str(got["rep"]), str(got["rep"])
+
+
+@pytest.mark.gpu
+def test_update_in_place_is_not_timed(tmp_path):
+    """The first call on a fresh lattice is a congrad whose M^dagger updates r in place (the
+    kernel chain): with the tuner on, the bits of the tuner turned off."""
+    _inputs(tmp_path, (8, 6, 4, 16), 0)
+    body = ("with thirring.Lattice(8, 6, 4, 16) as G:\n"
+            "    G.set_links(u); G._L.thr_profile(G.h, 1 << 20, 1)\n"
+            "    X = np.zeros_like(R); r['it'] = G.congrad(R, X, 0.2, 0.05, 3)[0]; r['x'] = X\n")
+    ref = _run(tmp_path, "ref", body, {"THR_TUNE": "0"})
+    got = _run(tmp_path, "alt", body, {"THR_TUNE": "1"})
+    assert int(ref["it"]) == int(got["it"]) and np.array_equal(ref["x"], got["x"])
