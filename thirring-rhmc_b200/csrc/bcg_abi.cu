@@ -228,6 +228,7 @@ int thr_pack_upload(thr_pack* k, int i, const double* u, const double* Phi, cons
   from_fortran_spinor<double2>(g, k->bb.B + E.off, st, k->st);
   THR_TRY(upload_fortran_spinor(g, st, X, k->st));
   from_fortran_spinor<double2>(g, k->bb.X + E.off, st, k->st);
+  THR_CUDA(cudaPeekAtLastError());
   THR_CUDA(cudaStreamSynchronize(k->st));
   return THR_OK;
 }

@@ -178,9 +178,11 @@ int upload_fortran_spinor(const Geom& g, double2* stage, const double* host, cud
   // page-locked arrays: without the t halos (2 of Lt + 2 planes; a pageable array goes through
   // the driver's staging buffers faster in one piece: 688 against 720 us at 18x14x10, Ls 20);
   // 2^31: the largest pitch a 2D copy takes
+  const bool pending = cudaPeekAtLastError() != cudaSuccess;  // an earlier launch's error: the caller's to report
   cudaPointerAttributes at;
-  const bool locked = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeHost;
-  if (!locked) cudaGetLastError();
+  const bool known = cudaPointerGetAttributes(&at, host) == cudaSuccess;
+  if (!known && !pending) cudaGetLastError();
+  const bool locked = known && at.type == cudaMemoryTypeHost;
   if (locked && pitch < (size_t)1 << 31) {
     e = cudaMemcpy2DAsync(reinterpret_cast<char*>(stage) + plane, pitch, reinterpret_cast<const char*>(host) + plane,
                           pitch, plane * g.lt, 4, cudaMemcpyHostToDevice, st);
