@@ -1,5 +1,6 @@
 """Switches that choose a schedule leave the results alone: the persistent multishift batch
-(THR_CHAIN) under the mixed solver's change of precision."""
+(THR_CHAIN) under the mixed solver's change of precision, the batched congrad without
+programmatic dependent launch (THR_PDL=0)."""
 import os
 import subprocess
 import sys
@@ -8,6 +9,7 @@ import numpy as np
 import pytest
 
 import oracle as O
+import thirring
 from helpers import rand_links, rand_spinor
 
 PKG = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "thirring-rhmc_b200")
@@ -51,3 +53,49 @@ def test_mixed_multishift_after_persistent_batches(tmp_path, chain):
     assert all(0 < ref["s" + k] < ref["i" + k] for k in ("12", "13", "22", "23"))
     for k in ref.files:
         assert np.array_equal(ref[k], got[k]), k
+
+
+@pytest.mark.gpu
+def test_batched_congrad_without_dependent_launches(tmp_path):
+    """Right-hand sides on one lattice and a pack of uneven lattices, FP64 and FP32 corrections:
+    THR_PDL=0 gives the bits and counts of the dependent launches and makes none of them
+    (launches with attributes go through cudaLaunchKernelExC, which a preloaded shim counts)."""
+    (tmp_path / "shim.c").write_text(
+        "#define _GNU_SOURCE\n#include <dlfcn.h>\n#include <stddef.h>\nint launches;\n"
+        "int cudaLaunchKernelExC(const void* cfg, const void* f, void** args) {\n"
+        "  static int (*next)(const void*, const void*, void**);\n"
+        "  if (!next) next = (int (*)(const void*, const void*, void**))dlsym(RTLD_NEXT, \"cudaLaunchKernelExC\");\n"
+        "  launches++;\n  return next(cfg, f, args);\n}\n")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(tmp_path / "shim.so"), str(tmp_path / "shim.c"), "-ldl"],
+                   check=True)
+    thirring.lib()
+    rt = next(v.split()[-1] for v in open("/proc/self/maps") if "libcudart" in v)
+    pre = {"LD_PRELOAD": "%s:%s" % (tmp_path / "shim.so", rt)}
+    dims, shapes = (6, 4, 8, 8), [(4, 4, 4, 8), (6, 4, 10, 20), (3, 5, 2, 33)]
+    rng = np.random.default_rng(19)
+    L = O.lat(*dims)
+    d = dict(u=rand_links(L, rng, beta=2.0), phi=np.stack([rand_spinor(L, rng) for _ in range(3)], axis=-1))
+    for i, s in enumerate(shapes):
+        Li = O.lat(*s)
+        d["u%d" % i], d["p%d" % i] = rand_links(Li, rng, beta=2.0), rand_spinor(Li, rng)
+    np.savez(tmp_path / "in.npz", **d)
+    body = ("import ctypes; shim = ctypes.CDLL(d + '/shim.so')\n"
+            "for mode in (thirring.FP64, thirring.MIXED_FP32):\n"
+            "    with thirring.Lattice(*%r) as G:\n"
+            "        G.set_links(ld('u')); x = np.zeros_like(ld('phi'))\n"
+            "        r['i%%d' %% mode], _ = G.congrad_multi(ld('phi'), x, 1e-6, 0.1, 3, mode)\n"
+            "        r['x%%d' %% mode] = x\n"
+            "    k = thirring.Pack(%r)\n"
+            "    for i in range(3):\n"
+            "        k.upload(i, ld('u%%d' %% i), ld('p%%d' %% i), np.zeros_like(ld('p%%d' %% i)))\n"
+            "    r['pi%%d' %% mode], _ = k.congrad(1e-6, 0.1, 1, mode)\n"
+            "    for i in range(3):\n"
+            "        r['p%%d%%d' %% (mode, i)] = k.download(i)\n"
+            "    k.close()\n"
+            "r['launches'] = ctypes.c_int.in_dll(shim, 'launches').value\n" % (dims, shapes))
+    ref = _run(tmp_path, "ref", body, pre)
+    got = _run(tmp_path, "alt", body, dict(pre, THR_PDL="0"))
+    assert ref["launches"] > 0 and got["launches"] == 0
+    for k in ref.files:
+        if k != "launches":
+            assert np.array_equal(ref[k], got[k]), k

@@ -24,6 +24,7 @@ struct BcgRun {
   const double2* u64 = nullptr;  // links, FP64 (packed per entry or shared)
   const void* ulow = nullptr;    // links, FP32
   int grid = 0;                  // persistent stencil grid (0 = default)
+  bool pdl = true;               // the three-kernel step as programmatic dependents
   BcgState* state = nullptr;     // [nent]
   int* skip = nullptr;           // [2 nent]: skip, and its copy the x and p update reads
   double* partials = nullptr;    // >= max(2 total_blocks, 64 * nent)

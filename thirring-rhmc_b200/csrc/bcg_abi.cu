@@ -2,6 +2,7 @@
 // context's lattice (thr_congrad_multi*) and many independent lattices of
 // uneven sizes packed together (thr_pack_*).
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
@@ -79,6 +80,7 @@ struct thr_pack {
   std::vector<Geom> geoms;
   BatchBufs bb;
   bool links_ready = false;
+  bool use_pdl = true;  // THR_PDL=0: off, as a context's
   long long launches = 0;
 };
 
@@ -88,8 +90,8 @@ Geom geom_of(const thr_params& p) {
 }
 size_t nf5_of(const Geom& g) { return (size_t)(g.ls + 2) * (g.lx + 2) * (g.ly + 2) * (g.lt + 2) * 4; }
 
-int run_batch(BatchBufs& bb, cudaStream_t st, int kernel, float am3, const double2* u64, const void* u32, float res,
-              float am, int imass, int precision, int* itercg, int* outer, long long* launches) {
+int run_batch(BatchBufs& bb, cudaStream_t st, bool pdl, int kernel, float am3, const double2* u64, const void* u32,
+              float res, float am, int imass, int precision, int* itercg, int* outer, long long* launches) {
   if (precision != THR_FP64 && precision != THR_MIXED_FP32 && precision != THR_MIXED_BF16) return THR_ERR_BADARG;
   BcgRun br;
   br.tab = &bb.tab;
@@ -98,6 +100,7 @@ int run_batch(BatchBufs& bb, cudaStream_t st, int kernel, float am3, const doubl
   br.am3 = am3;
   br.imass = imass;
   br.st = st;
+  br.pdl = pdl;
   br.u64 = u64;
   br.ulow = u32;
   br.state = bb.state;
@@ -138,8 +141,8 @@ int thr_congrad_multi_dev(thr_ctx* c, const void* Phi, void* X, int nrhs, float 
   const size_t bytes = (size_t)bb.tab.total_elems * sizeof(double2);
   THR_CUDA(cudaMemcpyAsync(bb.B, Phi, bytes, cudaMemcpyDeviceToDevice, c->st));
   THR_CUDA(cudaMemcpyAsync(bb.X, X, bytes, cudaMemcpyDeviceToDevice, c->st));
-  int rc = run_batch(bb, c->st, c->p.kernel, c->p.am3, c->u64, c->u32, res, am, imass, precision, itercg, outer,
-                     nullptr);
+  int rc = run_batch(bb, c->st, c->use_pdl, c->p.kernel, c->p.am3, c->u64, c->u32, res, am, imass, precision, itercg,
+                     outer, nullptr);
   if (rc != THR_OK && rc != THR_ERR_MAXITER) return rc;
   THR_CUDA(cudaMemcpyAsync(X, bb.X, bytes, cudaMemcpyDeviceToDevice, c->st));
   THR_CUDA(cudaStreamSynchronize(c->st));
@@ -161,8 +164,8 @@ int thr_congrad_multi(thr_ctx* c, const double* Phi, double* X, int nrhs, float 
     THR_TRY(c->upload_spinor(bb.B + k * n, Phi + 2 * nf * k));
     THR_TRY(c->upload_spinor(bb.X + k * n, X + 2 * nf * k));
   }
-  int rc = run_batch(bb, c->st, c->p.kernel, c->p.am3, c->u64, c->u32, res, am, imass, precision, itercg, outer,
-                     nullptr);
+  int rc = run_batch(bb, c->st, c->use_pdl, c->p.kernel, c->p.am3, c->u64, c->u32, res, am, imass, precision, itercg,
+                     outer, nullptr);
   if (rc != THR_OK && rc != THR_ERR_MAXITER) return rc;
   for (int k = 0; k < nrhs; k++) THR_TRY(c->download_spinor(X + 2 * nf * k, bb.X + k * n));
   int rs = c->sync();
@@ -175,6 +178,8 @@ int thr_pack_create(int n, const thr_params* p, int device, thr_pack** out) {
   *out = nullptr;
   thr_pack* k = new thr_pack();
   k->dev = device;
+  const char* e = std::getenv("THR_PDL");
+  if (e && e[0] == '0') k->use_pdl = false;
   if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&k->st, cudaStreamNonBlocking) != cudaSuccess) {
     delete k;
     return THR_ERR_CUDA;
@@ -238,8 +243,8 @@ int thr_pack_congrad(thr_pack* k, float res, float am, int imass, int precision,
   if (imass != 1 && imass != 3 && imass != 5) return THR_ERR_BADARG;
   cudaSetDevice(k->dev);
   const thr_params& p0 = k->p[0];
-  return run_batch(k->bb, k->st, p0.kernel, p0.am3, k->bb.u64, k->bb.u32, res, am, imass, precision, itercg, outer,
-                   &k->launches);
+  return run_batch(k->bb, k->st, k->use_pdl, p0.kernel, p0.am3, k->bb.u64, k->bb.u32, res, am, imass, precision,
+                   itercg, outer, &k->launches);
 }
 
 int thr_pack_download(thr_pack* k, int i, double* X) {

@@ -275,11 +275,11 @@ __global__ void __launch_bounds__(b_threads(PAIR), PAIR ? 6 : 3) k_bxp(BStep<S> 
 
 // MB, MD: resident blocks per SM of the M and the (larger) M^dagger blocks
 template <class S, bool PAIR, int MB, int MD>
-void launch_step(const BStep<S>& a, int blocks, cudaStream_t st) {
+void launch_step(const BStep<S>& a, int blocks, cudaStream_t st, bool pdl) {
   constexpr int kThr = b_threads(PAIR);
-  launch_k(k_bstencil<S, false, PAIR, MB>, dim3(blocks), dim3(kThr), 0, st, true, a);
-  launch_k(k_bstencil<S, true, PAIR, MD>, dim3(blocks), dim3(kThr + 32), 0, st, true, a);
-  launch_k(k_bxp<S, PAIR>, dim3(blocks), dim3(kThr), 0, st, true, a);
+  launch_k(k_bstencil<S, false, PAIR, MB>, dim3(blocks), dim3(kThr), 0, st, pdl, a);
+  launch_k(k_bstencil<S, true, PAIR, MD>, dim3(blocks), dim3(kThr + 32), 0, st, pdl, a);
+  launch_k(k_bxp<S, PAIR>, dim3(blocks), dim3(kThr), 0, st, pdl, a);
 }
 }  // namespace
 
@@ -306,18 +306,18 @@ int launch_bcg_step(BcgRun& br, VA* r, VS* p, VS* h, VA* e, int step, int inner_
   a.step = step;
   a.cap = inner_cap;
   if constexpr (sizeof(VS) == sizeof(float2)) {
-    if (t.even_ls) launch_step<VS, true, 8, 6>(a, t.total_blocks, br.st);
-    else launch_step<VS, false, 3, 3>(a, t.total_blocks, br.st);
+    if (t.even_ls) launch_step<VS, true, 8, 6>(a, t.total_blocks, br.st, br.pdl);
+    else launch_step<VS, false, 3, 3>(a, t.total_blocks, br.st, br.pdl);
   } else {
     // as many registers as do not cost a wave of blocks against four per SM.  FP64, us per
     // iteration with 2 / 3 / 4 per SM: 156 blocks 16.7 / 17.9 / 16.8; 432 - / 20.3 / 22.4; 512 - /
     // 28.5 / 25.1; 648 - / 30.6 / 31.4; 1145 - / 46.9 / 43.1; 1832 89 / 79 / 76.5
     const int sms = device_sms();
     auto waves = [&](int per) { return (t.total_blocks + per * sms - 1) / (per * sms); };
-    if (t.total_blocks <= sms) launch_step<VS, false, 1, 1>(a, t.total_blocks, br.st);
-    else if (waves(2) == waves(4)) launch_step<VS, false, 2, 2>(a, t.total_blocks, br.st);
-    else if (waves(3) == waves(4)) launch_step<VS, false, 3, 3>(a, t.total_blocks, br.st);
-    else launch_step<VS, false, 4, 4>(a, t.total_blocks, br.st);
+    if (t.total_blocks <= sms) launch_step<VS, false, 1, 1>(a, t.total_blocks, br.st, br.pdl);
+    else if (waves(2) == waves(4)) launch_step<VS, false, 2, 2>(a, t.total_blocks, br.st, br.pdl);
+    else if (waves(3) == waves(4)) launch_step<VS, false, 3, 3>(a, t.total_blocks, br.st, br.pdl);
+    else launch_step<VS, false, 4, 4>(a, t.total_blocks, br.st, br.pdl);
   }
   return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
 }
