@@ -97,3 +97,22 @@ def test_update_in_place_is_not_timed(tmp_path):
     ref = _run(tmp_path, "ref", body, {"THR_TUNE": "0"})
     got = _run(tmp_path, "alt", body, {"THR_TUNE": "1"})
     assert int(ref["it"]) == int(got["it"]) and np.array_equal(ref["x"], got["x"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("env", [{"THR_GRAPHS": "0"}, {}])
+@pytest.mark.parametrize("kernel,dims", [(0, (16, 16, 10, 65)), (1, (8, 6, 4, 16))])
+def test_congrad_chain_is_tuned(tmp_path, kernel, dims, env):
+    """A fresh lattice whose first call is a congrad in the kernel chain (above the lattices
+    with kernels of their own, or the Wilson operator), launched from the host or as a graph:
+    the tuner has settled both stencils, M^dagger's update among them; the bits of the tuner
+    turned off."""
+    _inputs(tmp_path, dims, kernel)
+    body = ("with thirring.Lattice(*%r, kernel=%d) as G:\n"
+            "    G.set_links(u); X = np.zeros_like(R); r['it'] = G.congrad(R, X, 0.2, 0.05, 3)[0]; r['x'] = X\n"
+            % (dims, kernel))
+    ref = _run(tmp_path, "ref", body, dict(env, THR_TUNE="0"))
+    got = _run(tmp_path, "alt", body, dict(env, THR_TUNE="1"))
+    assert int(ref["it"]) == int(got["it"]) > 2 and np.array_equal(ref["x"], got["x"])
+    for line in ("M epi=2", "Mdag epi=1"):
+        assert "fp64 %s %s %dx%dx%d Ls=%d " % (("wilson" if kernel else "shamir", line) + dims) in str(got["rep"]), line

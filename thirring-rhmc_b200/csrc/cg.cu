@@ -172,6 +172,20 @@ int cg_enqueue_chunk(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* r
   return cudaPeekAtLastError() == cudaSuccess ? THR_OK : THR_ERR_CUDA;
 }
 
+// The chain's two stencils once on separate fields (x1, x2 and the partials are scratch), so
+// that the tuner settles them: before a graph bakes them in, and before a host-launched chunk
+// updates r in place, which is never timed
+int cg_settle(thr_ctx* c, CgState* cs, const double2* p, const double2* r, double2* x1, double2* x2, float am,
+              int imass) {
+  if (c->cg_settled) return THR_OK;
+  THR_TRY(launch_dslash_norm<double2>(c->g, c->p.kernel, false, x1, p, c->u64, am, imass, c->p.am3, c->st, &cs->done,
+                                      c->partials));
+  THR_TRY(launch_dslash_axpy<double2>(c->g, c->p.kernel, true, x2, x1, c->u64, am, imass, c->p.am3, c->st, &cs->done,
+                                      r, &cs->nalpha, c->partials, c->rev_sweep ? 1 : 0));
+  c->cg_settled = true;
+  return THR_OK;
+}
+
 // The chunk loop as one CUDA graph (WHILE node), cached per buffers and operator.
 struct CgGraph {
   cudaGraph_t graph = nullptr;
@@ -214,12 +228,7 @@ int cg_graph_build(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* r, 
     return THR_OK;
   }
   G.release();
-  // the iteration's two stencils once outside the capture, so that the autotuner
-  // settles their configuration first (x1, x2 and the partials are scratch here)
-  THR_TRY(launch_dslash_norm<double2>(c->g, c->p.kernel, false, x1, p, c->u64, am, imass, c->p.am3, c->st, &cs->done,
-                                      c->partials));
-  THR_TRY(launch_dslash_axpy<double2>(c->g, c->p.kernel, true, x2, x1, c->u64, am, imass, c->p.am3, c->st, &cs->done,
-                                      r, &cs->nalpha, c->partials, c->rev_sweep ? 1 : 0));
+  THR_TRY(cg_settle(c, cs, p, r, x1, x2, am, imass));
   THR_CUDA(cudaGraphCreate(&G.graph, 0));
   cudaGraphConditionalHandle handle;
   THR_CUDA(cudaGraphConditionalHandleCreate(&handle, G.graph, 1, cudaGraphCondAssignDefault));
@@ -283,6 +292,7 @@ int congrad_dev(thr_ctx* c, const double2* Phi, double2* X, float res, float am,
     THR_CUDA(cudaMemcpyAsync(&h, cs, sizeof(CgState), cudaMemcpyDeviceToHost, c->st));
     THR_CUDA(cudaStreamSynchronize(c->st));
   } else {
+    THR_TRY(cg_settle(c, cs, p, r, x1, x2, am, imass));
     for (int base = 0; base < niterc + kCgChunk; base += kCgChunk) {
       THR_TRY(cg_enqueue_chunk(c, cs, X, p, r, x1, x2, am, imass));
       THR_CUDA(cudaMemcpyAsync(&h, cs, sizeof(CgState), cudaMemcpyDeviceToHost, c->st));
