@@ -116,3 +116,27 @@ def test_congrad_chain_is_tuned(tmp_path, kernel, dims, env):
     assert int(ref["it"]) == int(got["it"]) > 2 and np.array_equal(ref["x"], got["x"])
     for line in ("M epi=2", "Mdag epi=1"):
         assert "fp64 %s %s %dx%dx%d Ls=%d " % (("wilson" if kernel else "shamir", line) + dims) in str(got["rep"]), line
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("algo", [1, 2])
+def test_small_lattice_solves_tune_nothing(tmp_path, algo):
+    """Congrad and the multishift (FP64, FP32) on a lattice that runs the kernels with the
+    scalar steps inside: the stencils of the kernel chains are not launched, so neither are
+    their candidates; timing kernels runs the chains, tuned."""
+    _inputs(tmp_path, (6, 4, 4, 8), 0)
+    body = ("a = np.array([1e-2, 1.0])\n"
+            "def solve():\n"
+            "    G.set_links(u); X = np.zeros_like(R); G.congrad(R, X, 0.2, 0.05, 3)\n"
+            "    for sp in (False, True):\n"
+            "        G.multishift_solver(u, 0.05, 3, a, a, R, 1e-3, 100, sp=sp)\n"
+            "def report():\n"
+            "    b = C.create_string_buffer(1 << 16); thirring.lib().thr_tune_report(b, len(b))\n"
+            "    return b.value.decode()\n"
+            "with thirring.Lattice(6, 4, 4, 8, ndiag=2) as G:\n"
+            "    G.set_solver(%d); solve(); r['plain'] = report(); G._L.thr_profile(G.h, 1, 1); solve()\n" % algo)
+    out = _run(tmp_path, "out", body, {"THR_TUNE": "1"})
+    assert str(out["plain"]) == ""
+    for line in ("fp64 shamir M epi=2", "fp64 shamir M epi=3", "fp64 shamir Mdag epi=1", "fp32 shamir M epi=3",
+                 "fp32 shamir Mdag epi=1"):
+        assert line in str(out["rep"]), line

@@ -106,7 +106,10 @@ struct thr_ctx {
   double mixed_switch[2] = {1e-8, 1e-13};
   int mixed_switched_at = 0;  // iteration the last mixed solve left FP64 at (0: never)
   void* cg_graph = nullptr;  // cached congrad graph
-  bool cg_settled = false;   // the tuner has seen congrad's stencils (cg_settle)
+  // the tuner has seen the stencils of the kernel chains: congrad's (cg_settle), the batched
+  // multishift's in FP64, FP32 and BF16 storage (settle_stencils)
+  bool cg_settled = false;
+  bool ms_settled[3] = {};
   // sweep directions of the solver kernels (THR_REVERSE=0|1|2): 0 all bottom up; 1 the
   // M^dagger-with-update stencil top down; 2 (default) directions alternate per iteration
   // so each kernel starts on the sites its predecessor wrote last

@@ -314,6 +314,12 @@ void enqueue_flush(thr_ctx* c, cudaStream_t on, MsState* ms, MsHist* hist, MsCoe
   k_reset<<<1, 1, 0, on>>>(hist, ms);
 }
 
+// whether batches with base storage V run in steps.cu's kernels (except while kernels are timed)
+template <class V>
+bool batch_steps(const thr_ctx* c) {
+  return sizeof(V) >= sizeof(float2) && steps_apply(c, sizeof(V) == sizeof(double2));
+}
+
 // One batch of kBatch iterations on ring half `half` (stream order on `main`),
 // recording into hist[half]; alongside it, on c->st2, the flush of the batch
 // before (hist[1 - half], the other half).  Ring slots: iteration j of the batch
@@ -363,7 +369,7 @@ int enqueue_batch(thr_ctx* c, MsState* ms, MsHist* hist, MsCoef* cf, VO* out, VO
   }
   // small lattices (FP64 and FP32): two kernels per iteration, the scalar steps inside (steps.cu)
   constexpr bool can_step = sizeof(V) >= sizeof(float2);
-  const bool steps = can_step && !prof && steps_apply(c, fp64);
+  const bool steps = !prof && batch_steps<V>(c);
   for (int j = 0; j < kBatch; j++) {
     const int so = half * kBatch + j, sn = so + 1 == 2 * kBatch ? 0 : so + 1;
     V* rold = ring + (size_t)so * n;
@@ -429,6 +435,22 @@ template <class V, class VO> constexpr int graph_slot() {
   return sizeof(VO) == sizeof(float2) ? 1 : sizeof(V) == sizeof(double2) ? 0 : sizeof(V) == sizeof(float2) ? 2 : 3;
 }
 
+// The chain's two stencils once, so that the tuner settles them: before a graph bakes them in,
+// and before launches are timed (hv, p, s and the partials are scratch at this point; the
+// solve clears hv and p after); once per context and storage
+template <class V>
+int settle_stencils(thr_ctx* c, MsState* ms, V* ring, V* p, V* hv, V* s, float am, int imass) {
+  bool& settled = c->ms_settled[sizeof(V) == sizeof(double2) ? 0 : sizeof(V) == sizeof(float2) ? 1 : 2];
+  if (settled) return THR_OK;
+  const auto* u = (const typename Sto<V>::C*)(sizeof(V) == sizeof(double2) ? (const void*)c->u64 : (const void*)c->u32);
+  THR_TRY(launch_dslash_accum<V>(c->g, c->p.kernel, false, hv, ring, u, am, imass, c->p.am3, c->st, &ms->done, p,
+                                 &ms->gammag, c->partials, 0));
+  THR_TRY(launch_dslash_axpy<V>(c->g, c->p.kernel, true, s, hv, u, am, imass, c->p.am3, c->st, &ms->done, ring,
+                                &ms->omega, c->partials, c->rev_sweep ? 1 : 0));
+  settled = true;
+  return THR_OK;
+}
+
 template <class V, class VO = V>
 int ms_graph_build(thr_ctx* c, MsState* ms, MsHist* hist, MsCoef* cf, VO* out, VO* sf, V* ring, V* p, V* hv, V* s,
                    float am, int imass, cudaGraphExec_t* exec_out);
@@ -466,16 +488,7 @@ int ms_graph_build(thr_ctx* c, MsState* ms, MsHist* hist, MsCoef* cf, VO* out, V
     return THR_OK;
   }
   G.release();
-  // run the two stencils of an iteration once outside the capture, so that the
-  // autotuner settles their configuration before it is baked into the graph
-  // (hv, p, s and the partials are scratch at this point; the solve clears hv and p after)
-  {
-    const typename Sto<V>::C* uu = (const typename Sto<V>::C*)u;
-    THR_TRY(launch_dslash_accum<V>(c->g, c->p.kernel, false, hv, ring, uu, am, imass, c->p.am3, c->st, &ms->done, p,
-                                   &ms->gammag, c->partials, 0));
-    THR_TRY(launch_dslash_axpy<V>(c->g, c->p.kernel, true, s, hv, uu, am, imass, c->p.am3, c->st, &ms->done, ring,
-                                  &ms->omega, c->partials, c->rev_sweep ? 1 : 0));
-  }
+  if (!batch_steps<V>(c)) THR_TRY(settle_stencils<V>(c, ms, ring, p, hv, s, am, imass));
   THR_CUDA(cudaGraphCreate(&G.graph, 0));
   cudaGraphConditionalHandle handle;
   THR_CUDA(cudaGraphConditionalHandleCreate(&handle, G.graph, 1, cudaGraphCondAssignDefault));
@@ -598,6 +611,7 @@ int run_batches(thr_ctx* c, MsState* ms, MsState* h, MsHist* hist, MsCoef* cf, V
     return THR_OK;
   }
   // stream-launched batches, one synchronisation per batch (and kernel timing)
+  if (c->prof_on) THR_TRY(settle_stencils<V>(c, ms, ring, p, hv, s, am, imass));
   THR_TRY(prime());
   const size_t prof_first = c->prof_kind.size();
   THR_CUDA(cudaMemcpyAsync(h, ms, sizeof(MsState), cudaMemcpyDeviceToHost, c->st));
