@@ -147,7 +147,7 @@ int cg_enqueue_chunk(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* r
   // chunk's first, which follows the loop control, excepted; THR_PDL=0: none); each waits
   // for its predecessor before it reads anything, so the results are the same
   const bool pdl = c->use_pdl;
-  const bool steps = !c->prof_on && steps_apply(c);  // the chain while kernels are timed, as the multishift
+  const bool steps = !c->prof_on && cg_steps_apply(c);  // the chain while kernels are timed, as the multishift
   for (int k = 0; k < kCgChunk; k++) {
     // sweep directions alternate with the iteration's parity (kCgChunk is even): each
     // kernel starts on the sites its predecessor wrote last (results do not depend on it)
@@ -228,7 +228,7 @@ int cg_graph_build(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* r, 
     return THR_OK;
   }
   G.release();
-  if (!steps_apply(c)) THR_TRY(cg_settle(c, cs, p, r, x1, x2, am, imass));
+  if (!cg_steps_apply(c)) THR_TRY(cg_settle(c, cs, p, r, x1, x2, am, imass));
   THR_CUDA(cudaGraphCreate(&G.graph, 0));
   cudaGraphConditionalHandle handle;
   THR_CUDA(cudaGraphConditionalHandleCreate(&handle, G.graph, 1, cudaGraphCondAssignDefault));
@@ -292,7 +292,7 @@ int congrad_dev(thr_ctx* c, const double2* Phi, double2* X, float res, float am,
     THR_CUDA(cudaMemcpyAsync(&h, cs, sizeof(CgState), cudaMemcpyDeviceToHost, c->st));
     THR_CUDA(cudaStreamSynchronize(c->st));
   } else {
-    if (c->prof_on || !steps_apply(c)) THR_TRY(cg_settle(c, cs, p, r, x1, x2, am, imass));
+    if (c->prof_on || !cg_steps_apply(c)) THR_TRY(cg_settle(c, cs, p, r, x1, x2, am, imass));
     for (int base = 0; base < niterc + kCgChunk; base += kCgChunk) {
       THR_TRY(cg_enqueue_chunk(c, cs, X, p, r, x1, x2, am, imass));
       THR_CUDA(cudaMemcpyAsync(&h, cs, sizeof(CgState), cudaMemcpyDeviceToHost, c->st));

@@ -317,7 +317,7 @@ void enqueue_flush(thr_ctx* c, cudaStream_t on, MsState* ms, MsHist* hist, MsCoe
 // whether batches with base storage V run in steps.cu's kernels (except while kernels are timed)
 template <class V>
 bool batch_steps(const thr_ctx* c) {
-  return sizeof(V) >= sizeof(float2) && steps_apply(c, sizeof(V) == sizeof(double2));
+  return sizeof(V) >= sizeof(float2) && ms_steps_apply(c, sizeof(V) == sizeof(double2));
 }
 
 // One batch of kBatch iterations on ring half `half` (stream order on `main`),

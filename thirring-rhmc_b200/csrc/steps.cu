@@ -12,9 +12,14 @@
 // The sums run in block_sum_partials' order, the stencils and the recurrences are the
 // kernel chain's, so the bits are the same.  Measured at 12^2x12, Ls 16 (216 blocks): 7.5 us
 // per iteration instead of 14.0 (7.9 with the state advanced by a stencil block, 9.8 while
-// its copy took a round trip per four rows and every warp waited for the flag first).  Every
-// block reads every partial, so lattices of more than kStepMaxParts blocks keep the chain
-// (there its one-block sums are 5 us of 100).
+// its copy took a round trip per four rows and every warp waited for the flag first).
+//
+// Every block reads every partial and holds its epilogue until the sum is known, which pays
+// while the grid is one wave (kMsStepPerSm).  us per multishift iteration, FP64 / FP32, these
+// kernels against the chain (one B200): 549 blocks (14^3, Ls 24) 11.4 / 10.6 against 16.4 / 14.2;
+// 729 (18^3, Ls 16) 15.5 / 10.9, 17.5 / 16.2; 880 (22x20x16, Ls 16) 19.0 / 13.4, 19.7 / 16.3; and
+// past one wave 896 (16^2x14, Ls 32) 21.1 / 17.5 against 19.8 / 16.6; 1331 (22^3, Ls 16) 32.0 /
+// 21.1, 25.6 / 18.7; 2048 (32^3, Ls 8) 45.6 / 31.9, 33.0 / 22.8.
 //
 // Nothing a kernel reads is written by it: the sums' input and output partials alternate
 // between two arrays, the M step reads delta from dl[] of one parity and writes the other,
@@ -24,7 +29,9 @@
 // Congrad's iteration is three kernels instead of six in the same way: M p, the M^dagger
 // step with alpha inside, and the x and p update with beta inside (pending_done, set by the
 // update, is read by the stencils; done, set by the M^dagger step, by the update).  At
-// 12^2x12, Ls 16: 10.7 us per iteration instead of 17.5.
+// 12^2x12, Ls 16: 10.7 us per iteration instead of 17.5; its third kernel has the sum ahead of
+// a pass over memory, so the line is lower (kCgStepPerSm): 549 blocks 16.6 against 21.3, 729
+// 21.8 / 22.6, 768 (16^2x12, Ls 32) 23.0 / 23.0, 880 26.1 / 24.3, 1331 40.0 / 32.3.
 #include <algorithm>
 #include <type_traits>
 
@@ -39,11 +46,13 @@ namespace thr {
 namespace {
 constexpr int kStepThreads = 128;                   // the Shamir stencil's blocks
 constexpr int kStepBlock = kStepThreads + 32;       // and the scalar warp
-constexpr int kStepMaxParts = 2048;                 // two partials per virtual thread of the sum
+constexpr int kStepMaxParts = 1024;                 // one partial per virtual thread of the sum
+// blocks per SM up to which the kernels are taken, the lead block included
+constexpr int kMsStepPerSm = 6, kCgStepPerSm = 5;
 
-// sum of p[0..n) (n <= 2048) in every lane of one warp, as block_sum_partials adds them
-// with 1024 threads: thread i adds p[i] and p[i + 1024], each warp's 32 values go through a
-// halving tree, then the 32 warp sums.  A butterfly gives the tree's value (lane 0 of the
+// sum of p[0..n) (n <= 1024) in every lane of one warp, as block_sum_partials adds them
+// with 1024 threads: thread i has p[i], each warp's 32 values go through a halving tree, then
+// the 32 warp sums.  A butterfly gives the tree's value (lane 0 of the
 // tree; the operands of an addition commute) in all lanes.
 __device__ __forceinline__ double warp_sum_partials(const double* p, int n, int lane) {
   constexpr int kU = 8;  // virtual warps in flight
@@ -54,13 +63,6 @@ __device__ __forceinline__ double warp_sum_partials(const double* p, int n, int 
     for (int k = 0; k < kU; k++) {
       const int i = (w0 + k) * 32 + lane;
       v[k] = i < n ? p[i] : 0.0;
-    }
-    if (n > 1024) {
-#pragma unroll
-      for (int k = 0; k < kU; k++) {
-        const int i = (w0 + k) * 32 + lane + 1024;
-        if (i < n) v[k] += p[i];
-      }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -409,26 +411,26 @@ StepArgs<C> step_args(thr_ctx* c, C* out, const C* in, const C* aux, float am, i
 
 constexpr int kStepMaxShflBudget = 4;
 
-// launch(integral_constant<int, MB>): the resident blocks per SM that a kernel's registers are
-// budgeted for.  One wave of blocks with as many registers as that leaves (a site's loads in
-// flight at once); a grid of more than six blocks per SM runs in several waves anyway, and
-// four keep its loads together.  FP64 multishift, us per iteration with budgets 2 to 6 (the
+// launch(integral_constant<int, MB>): the resident blocks per SM (2 to MOST) that a kernel's
+// registers are budgeted for: one wave of blocks with as many registers as that leaves (a
+// site's loads in flight at once).  FP64 multishift, us per iteration with budgets 2 to 6 (the
 // rule's marked): 343 blocks (14^3, Ls 16) 12.6 [8.5] 10.4 12.1 14.8; 549 (14^3, Ls 24) 15.9 16.4
 // [12.2] 13.3 15.5; 683 (16^3, Ls 20) 20.8 17.2 18.6 [15.2] 16.4; 820 (16^3, Ls 24) 23.5 19.5 20.3
-// 22.5 [18.1]; 1000 (20^3, Ls 16) 29.0 25.5 [22.1] 25.0 31.7.  Congrad's stencils alike (343: 13.8
-// [12.9] 14.3 15.2 17.4; 683: 24.0 22.4 23.3 [19.7] 21.1).
-// Up to four blocks s -+ 1 comes by shuffles where Ls allows it (343 blocks: 8.5 against 9.4);
-// in the registers that five or six leave they spill, and the neighbours are read (729 blocks,
-// 18^3, Ls 16: 15.3 against 16.9; 800, 20^2 x 16, Ls 16: 18.2 against 24.0).
-template <class F>
+// 22.5 [18.1].  Congrad's stencils alike (343: 13.8 [12.9] 14.3 15.2 17.4; 683: 24.0 22.4 23.3
+// [19.7] 21.1).
+// Up to four blocks s -+ 1 comes by shuffles where Ls allows it (343 blocks: 8.5 against 9.4; at
+// four the M^dagger kernels with shuffles spill 20 bytes); in the registers that five or six
+// leave they spill more, and the neighbours are read (729 blocks, 18^3, Ls 16: 15.3 against
+// 16.9; 800, 20^2 x 16, Ls 16: 18.2 against 24.0).
+template <int MOST, class F>
 void with_budget(int blocks, F&& launch) {
   using std::integral_constant;
   const int sms = device_sms();
   if (blocks <= 2 * sms) launch(integral_constant<int, 2>{});
   else if (blocks <= 3 * sms) launch(integral_constant<int, 3>{});
-  else if (blocks <= 4 * sms || blocks > 6 * sms) launch(integral_constant<int, 4>{});
-  else if (blocks <= 5 * sms) launch(integral_constant<int, 5>{});
-  else launch(integral_constant<int, 6>{});
+  else if (blocks <= 4 * sms) launch(integral_constant<int, 4>{});
+  else if (MOST == 5 || blocks <= 5 * sms) launch(integral_constant<int, 5>{});
+  else if constexpr (MOST > 5) launch(integral_constant<int, MOST>{});
 }
 
 template <class C, int PER, bool DAG>
@@ -445,7 +447,7 @@ void launch_ms_step(const StepArgs<C>& a, MsState* ms, MsHist* rec, int j, cudaS
     launch_k(k_ms_step<C, PER, DAG, false, MB>, grd, blk, 0, st, pdl, a, ms, rec, j);
   };
   if constexpr (PER == 1) {
-    with_budget(a.np, go);
+    with_budget<kMsStepPerSm>(a.np, go);
   } else {  // blocks of 96 threads: six of them leave the registers a site needs
     if (a.np <= 2 * device_sms()) go(std::integral_constant<int, 2>{});
     else go(std::integral_constant<int, 6>{});
@@ -453,11 +455,14 @@ void launch_ms_step(const StepArgs<C>& a, MsState* ms, MsHist* rec, int j, cudaS
 }
 }  // namespace
 
-bool steps_apply(const thr_ctx* c, bool fp64) {
+static bool steps_apply(const thr_ctx* c, bool fp64, int per_sm) {
   const unsigned np = stencil_grid(c->g, 0);
   return c->p.kernel == 0 && c->g.ls <= kStepThreads && np <= (unsigned)kStepMaxParts &&
-         stencil_parts(c->g, 0, fp64) == np && 2 * (size_t)np + 2 <= c->nparts;
+         np + 1 <= (unsigned)(per_sm * device_sms()) && stencil_parts(c->g, 0, fp64) == np &&
+         2 * (size_t)np + 2 <= c->nparts;
 }
+bool ms_steps_apply(const thr_ctx* c, bool fp64) { return steps_apply(c, fp64, kMsStepPerSm); }
+bool cg_steps_apply(const thr_ctx* c) { return steps_apply(c, true, kCgStepPerSm); }
 
 double* steps_partials2(const thr_ctx* c) { return c->partials + ((stencil_grid(c->g, 0) + 1) & ~1u); }
 
@@ -489,7 +494,7 @@ int cg_step_iteration(thr_ctx* c, CgState* cs, double2* X, double2* p, double2* 
   double *pa = c->partials, *pb = steps_partials2(c);
   const StepArgs<double2> a = step_args<double2>(c, r, h, r, am, imass, pa, pb, rev_md);
   const StepArgs<double2> m = step_args<double2>(c, h, p, nullptr, am, imass, nullptr, pa, rev_m);
-  with_budget(a.np, [&](auto mb) {
+  with_budget<kCgStepPerSm>(a.np, [&](auto mb) {
     constexpr int MB = decltype(mb)::value;
     auto run = [&](auto sh) {
       constexpr bool SH = decltype(sh)::value;

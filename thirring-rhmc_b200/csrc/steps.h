@@ -7,8 +7,9 @@
 
 namespace thr {
 
-// whether the context's lattice takes them
-bool steps_apply(const thr_ctx* c, bool fp64 = true);
+// whether the context's lattice takes them (its device is current)
+bool ms_steps_apply(const thr_ctx* c, bool fp64);
+bool cg_steps_apply(const thr_ctx* c);
 // the second array of stencil partials (the first is c->partials)
 double* steps_partials2(const thr_ctx* c);
 
