@@ -35,7 +35,7 @@ struct BatchTable {
   bool even_ls = true;        // every entry's Ls is even
   std::vector<BatchEntry> host;
   BatchEntry* dev = nullptr;
-  int* wmap = nullptr;        // device: the entry of each work block
+  int* wmap = nullptr;        // device, behind dev's entries: the entry of each work block
   ~BatchTable();
   // shared_links: all entries use the links at offset 0 (right-hand sides of one lattice)
   int build(const std::vector<Geom>& geoms, bool shared_links, cudaStream_t st);

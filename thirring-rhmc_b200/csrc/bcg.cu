@@ -28,10 +28,7 @@
 
 namespace thr {
 
-BatchTable::~BatchTable() {
-  cudaFree(dev);
-  cudaFree(wmap);
-}
+BatchTable::~BatchTable() { cudaFree(dev); }
 
 int BatchTable::build(const std::vector<Geom>& geoms, bool shared_links, cudaStream_t st) {
   host.clear();
@@ -60,15 +57,16 @@ int BatchTable::build(const std::vector<Geom>& geoms, bool shared_links, cudaStr
     host.push_back(e);
   }
   cudaFree(dev);
-  cudaFree(wmap);
   dev = nullptr;
   wmap = nullptr;
-  if (cudaMalloc(&wmap, sizeof(int) * std::max(1, total_blocks)) != cudaSuccess) return THR_ERR_NOMEM;
-  if (cudaMemcpyAsync(wmap, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice, st) != cudaSuccess)
-    return THR_ERR_CUDA;
-  if (cudaMalloc(&dev, sizeof(BatchEntry) * std::max(1, nent)) != cudaSuccess) return THR_ERR_NOMEM;
-  if (cudaMemcpyAsync(dev, host.data(), sizeof(BatchEntry) * nent, cudaMemcpyHostToDevice, st) != cudaSuccess)
-    return THR_ERR_CUDA;
+  // one allocation and one copy: the entries, then the entry of each work block
+  const size_t tb = sizeof(BatchEntry) * (size_t)nent, bytes = tb + sizeof(int) * map.size();
+  std::vector<unsigned char> img(bytes);
+  std::copy_n(reinterpret_cast<const unsigned char*>(host.data()), tb, img.data());
+  std::copy_n(reinterpret_cast<const unsigned char*>(map.data()), bytes - tb, img.data() + tb);
+  if (cudaMalloc(&dev, std::max<size_t>(1, bytes)) != cudaSuccess) return THR_ERR_NOMEM;
+  wmap = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(dev) + tb);
+  if (cudaMemcpyAsync(dev, img.data(), bytes, cudaMemcpyHostToDevice, st) != cudaSuccess) return THR_ERR_CUDA;
   return THR_OK;
 }
 

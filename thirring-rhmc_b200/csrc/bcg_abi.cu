@@ -32,6 +32,7 @@ struct BatchBufs {
   size_t stage_bytes = 0;
   BcgState* hstate = nullptr;  // pinned
   cudaEvent_t ev[2] = {};
+  bool lent = false;           // hstate and ev are a context's
   ~BatchBufs() { release(); }
   void release() {
     for (void* ptr : {(void*)state, (void*)skip, (void*)partials, (void*)B, (void*)X, (void*)R, (void*)T, (void*)H, r,
@@ -39,21 +40,31 @@ struct BatchBufs {
       cudaFree(ptr);
     state = nullptr; skip = nullptr; partials = nullptr; B = X = R = T = H = nullptr;
     r = p = h = q = e = nullptr; u64 = nullptr; u32 = nullptr; stage = nullptr;
-    if (hstate) cudaFreeHost(hstate);
+    if (hstate && !lent) cudaFreeHost(hstate);
     hstate = nullptr;
     for (cudaEvent_t& v : ev) {
-      if (v) cudaEventDestroy(v);
+      if (v && !lent) cudaEventDestroy(v);
       v = nullptr;
     }
   }
-  int alloc(bool own_links, size_t stage_b) {
+  // c: the solve is one call on this context, which lends its pinned mirror where that is large
+  // enough and the flush's events (nothing else of the context runs meanwhile): a two-source
+  // solve on 4^3, Ls 8 that ends at once takes 149 us, 159 with its own and a table more
+  int alloc(bool own_links, size_t stage_b, thr_ctx* c = nullptr) {
     const size_t n = (size_t)tab.total_elems, ne = (size_t)tab.nent;
     const size_t nparts = std::max(2 * (size_t)tab.total_blocks, 64 * ne) + 64;
     bool ok = cudaMalloc(&state, sizeof(BcgState) * ne) == cudaSuccess &&
               cudaMalloc(&skip, sizeof(int) * 2 * ne) == cudaSuccess &&
-              cudaMalloc(&partials, sizeof(double) * nparts) == cudaSuccess &&
-              cudaMallocHost(&hstate, 2 * sizeof(BcgState) * ne) == cudaSuccess;
-    for (cudaEvent_t& v : ev) ok = ok && cudaEventCreateWithFlags(&v, cudaEventDisableTiming) == cudaSuccess;
+              cudaMalloc(&partials, sizeof(double) * nparts) == cudaSuccess;
+    lent = c && 2 * sizeof(BcgState) * ne <= kHostScalars * sizeof(double);
+    if (lent) {
+      hstate = reinterpret_cast<BcgState*>(c->hscal);
+      ev[0] = c->ev_fork[0];
+      ev[1] = c->ev_fork[1];
+    } else {
+      ok = ok && cudaMallocHost(&hstate, 2 * sizeof(BcgState) * ne) == cudaSuccess;
+      for (cudaEvent_t& v : ev) ok = ok && cudaEventCreateWithFlags(&v, cudaEventDisableTiming) == cudaSuccess;
+    }
     for (double2** f : {&B, &X, &R, &T, &H}) ok = ok && cudaMalloc(f, n * sizeof(double2)) == cudaSuccess;
     // the inner vectors are sized for FP64 so any precision fits
     for (void** f : {&r, &p, &h, &q, &e}) ok = ok && cudaMalloc(f, n * sizeof(double2)) == cudaSuccess;
@@ -137,7 +148,7 @@ int thr_congrad_multi_dev(thr_ctx* c, const void* Phi, void* X, int nrhs, float 
   BatchBufs bb;
   std::vector<Geom> gs(nrhs, c->g);
   THR_TRY(bb.tab.build(gs, true, c->st));
-  THR_TRY(bb.alloc(false, 0));
+  THR_TRY(bb.alloc(false, 0, c));
   const size_t bytes = (size_t)bb.tab.total_elems * sizeof(double2);
   THR_CUDA(cudaMemcpyAsync(bb.B, Phi, bytes, cudaMemcpyDeviceToDevice, c->st));
   THR_CUDA(cudaMemcpyAsync(bb.X, X, bytes, cudaMemcpyDeviceToDevice, c->st));
@@ -158,7 +169,7 @@ int thr_congrad_multi(thr_ctx* c, const double* Phi, double* X, int nrhs, float 
   BatchBufs bb;
   std::vector<Geom> gs(nrhs, c->g);
   THR_TRY(bb.tab.build(gs, true, c->st));
-  THR_TRY(bb.alloc(false, 0));
+  THR_TRY(bb.alloc(false, 0, c));
   const size_t n = c->n4(), nf = c->nf5();
   for (int k = 0; k < nrhs; k++) {
     THR_TRY(c->upload_spinor(bb.B + k * n, Phi + 2 * nf * k));

@@ -191,16 +191,16 @@ int thr_create(const thr_params* p, thr_ctx** out) {
   const size_t nparts = std::max<size_t>((size_t)kMaxPartials * 8, (size_t)std::max(stencil_grid(c->g, 0), stencil_grid(c->g, 1)) + 1024);
   if (!rc && cudaMalloc(&c->partials, nparts * sizeof(double)) != cudaSuccess) rc = THR_ERR_NOMEM;
   c->nparts = nparts;
-  if (!rc && cudaMalloc(&c->dscal, 4096 * sizeof(double)) != cudaSuccess) rc = THR_ERR_NOMEM;
+  if (!rc && cudaMalloc(&c->dscal, kHostScalars * sizeof(double)) != cudaSuccess) rc = THR_ERR_NOMEM;
   if (!rc && cudaMalloc(&c->iscal, 1024 * sizeof(int)) != cudaSuccess) rc = THR_ERR_NOMEM;
-  if (!rc && cudaMallocHost(&c->hscal, 4096 * sizeof(double)) != cudaSuccess) rc = THR_ERR_NOMEM;
+  if (!rc && cudaMallocHost(&c->hscal, kHostScalars * sizeof(double)) != cudaSuccess) rc = THR_ERR_NOMEM;
   if (!rc && cudaMallocHost(&c->hiscal, 1024 * sizeof(int)) != cudaSuccess) rc = THR_ERR_NOMEM;
   if (!rc && cudaMallocHost(&c->ms_tmpl, kMsTemplates * sizeof(MsState)) != cudaSuccess) rc = THR_ERR_NOMEM;
   if (rc) {
     thr_destroy(c);
     return rc;
   }
-  cudaMemsetAsync(c->dscal, 0, 4096 * sizeof(double), c->st);
+  cudaMemsetAsync(c->dscal, 0, kHostScalars * sizeof(double), c->st);
   cudaMemsetAsync(c->iscal, 0, 1024 * sizeof(int), c->st);
   *out = c;
   return THR_OK;

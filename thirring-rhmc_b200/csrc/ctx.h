@@ -20,7 +20,9 @@
     if (rc_ != THR_OK) return rc_;    \
   } while (0)
 
-// slots of the context's device scalar block (dscal, 4096 doubles) outside the
+// the context's device scalar block (dscal) and its pinned mirror (hscal), in doubles
+constexpr size_t kHostScalars = 4096;
+// slots of the scalar block outside the
 // solver states that start at its base
 constexpr int kScalHamSum = 4000;      // hamilton's fermion sum
 constexpr int kScalFusedCoef = 4090;   // thr_dslash_fused_dev: the epilogue coefficient
