@@ -1,5 +1,5 @@
 """Switches that choose a schedule leave the results alone: the persistent multishift batch
-(THR_CHAIN) under the mixed solver's change of precision, the batched congrad without
+(THR_CHAIN) under the mixed solver's change of precision and with the Wilson kernel, the batched congrad without
 programmatic dependent launch (THR_PDL=0)."""
 import os
 import subprocess
@@ -99,3 +99,31 @@ def test_batched_congrad_without_dependent_launches(tmp_path):
     for k in ref.files:
         if k != "launches":
             assert np.array_equal(ref[k], got[k]), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,layout,chain", [((4, 4, 6, 8), 0, "1"), ((4, 6, 6, 12), 1, "1"), ((5, 3, 4, 33), 0, "1"),
+                                               ((24, 24, 16, 16), 0, "2")])
+def test_wilson_persistent_batches(tmp_path, dims, layout, chain):
+    """The Wilson kernel's multishift in persistent batches: one block per site block, idle
+    threads, both site orders, and more site blocks than resident blocks; the bits and
+    counts of the kernel chain, stopped inside a batch.  That the persistent kernel runs
+    shows in its bounded barriers: told to wait for one arrival too many they run out and
+    the solve ends with THR_ERR_TIMEOUT (8)."""
+    rng = np.random.default_rng(47)
+    L = O.lat(*dims, kernel=1)
+    np.savez(tmp_path / "in.npz", u=rand_links(L, rng), phi=rand_spinor(L, rng))
+    body = ("a, b = np.array([1e-3, 0.05, 0.7, 30.0]), np.array([0.3, 0.5, 0.8, 2.0]); r['status'] = 0\n"
+            "with thirring.Lattice(*%r, kernel=1, layout=%d, ndiag=4) as G:\n"
+            "    try:\n"
+            "        r['x'], r['i'], r['c'] = G.multishift_solver(ld('u'), 0.05, 3, a, b, ld('phi'), 1e-9, 77)\n"
+            "    except thirring.ThirringError as e:\n"
+            "        r['status'] = e.status\n" % (dims, layout))
+    ref = _run(tmp_path, "ref", body, {"THR_CHAIN": "0"})
+    got = _run(tmp_path, "alt", body, {"THR_CHAIN": chain})
+    assert int(ref["status"]) == 0 and int(ref["i"]) == 77
+    for k in ref.files:
+        assert np.array_equal(ref[k], got[k]), k
+    if dims[0] == 4:
+        out = _run(tmp_path, "bound", body, {"THR_CHAIN": chain, "THR_CHAIN_WAIT_TEST": "1"})
+        assert int(out["status"]) == 8

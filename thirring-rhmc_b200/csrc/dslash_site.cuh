@@ -414,8 +414,8 @@ __device__ __forceinline__ void hop_halves(int mu, bool plus, C W, const C* r, C
 // One 5D site of the Wilson (OV false) or overlap (OV true) operator.  Every thread of the
 // block calls it (live false: a thread without a site); ex: NT x (DAG ? 4 : 8) values in
 // shared memory, read by nobody once every thread has returned from a __syncthreads().
-// tid - s .. tid - s + Ls - 1 are the threads of this thread's site.
-template <class S, bool OV, bool DAG, int NT>
+// tid - s .. tid - s + Ls - 1 are the threads of this thread's site.  COH: see sto_ld.
+template <class S, bool OV, bool DAG, int NT, bool COH = false>
 __device__ __forceinline__ void wilson_exchange(const S* __restrict__ in, const typename Sto<S>::C* __restrict__ u,
                                                 const Geom& g, int s, int site, bool live, int tid, float am,
                                                 int imass, float am3, const double* __restrict__ zc,
@@ -436,7 +436,7 @@ __device__ __forceinline__ void wilson_exchange(const S* __restrict__ in, const 
     const unsigned i0 = (unsigned)s + (unsigned)Ls * (unsigned)site;
 #pragma unroll
     for (int d = 0; d < 4; d++) {
-      r[d] = Sto<S>::ld(pl[d], i0);
+      r[d] = sto_ld<S, COH>(pl[d], i0);
       A[d] = B[d] = mk(R(0), R(0));
     }
     if (DAG) {
@@ -452,7 +452,7 @@ __device__ __forceinline__ void wilson_exchange(const S* __restrict__ in, const 
         const unsigned i = (unsigned)s + (unsigned)Ls * (unsigned)ns;
         C q[4];
 #pragma unroll
-        for (int d = 0; d < 4; d++) q[d] = Sto<S>::ld(pl[d], i);
+        for (int d = 0; d < 4; d++) q[d] = sto_ld<S, COH>(pl[d], i);
         if (DAG) hop_projected<C, R>(mu, dir != 0, W, q, A);
         else hop_halves<C>(mu, dir == 0, W, q, A, B);
       }
@@ -501,7 +501,7 @@ __device__ __forceinline__ void wilson_exchange(const S* __restrict__ in, const 
       const C v = (A[d] + B[d]) + ((inp ? fa : cmul(wp, fa)) + (inn ? gb : cmul(wn, gb)));
       if (OV) {
         const bool lo = d < 2;
-        const C n = Sto<S>::ld(pl[d], (unsigned)Ls * (unsigned)site +
+        const C n = sto_ld<S, COH>(pl[d], (unsigned)Ls * (unsigned)site +
                                           (unsigned)(lo ? (inp ? s - 1 : Ls - 1) : (inn ? s + 1 : 0)));
         const C wr = (lo ? inp : inn) ? n : cmul(lo ? wp : wn, n);
         res[d] = cs * v + r[d] - wr;

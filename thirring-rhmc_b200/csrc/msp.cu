@@ -78,7 +78,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, int
 // The partials of a stencil pass, written by every block, are copied into shared memory
 // with cp.async (16 bytes each, through L2) right after the barrier, while the block
 // computes its next stencil pass; the sum waits for them only when its result is due.
-constexpr int kChainThreads = 128;     // the Shamir stencil's blocks
+constexpr int kChainThreads = 128;    // the stencils' blocks
 constexpr int kChainMaxParts = 2048;  // partials one block stages (stencil site blocks)
 __device__ __forceinline__ void stage_partials(double* sp, const double* p, int n, int tid, int nthr) {
   const int n2 = (n + 1) & ~1;  // the arrays are padded to an even length
@@ -139,9 +139,10 @@ struct ChainArgs {
   unsigned extra;  // added to every barrier's target (the timeout test); 0 in use
 };
 
-template <bool SHFL>
+template <int KER, bool SHFL>
 __global__ void __launch_bounds__(kChainThreads, 512 / kChainThreads) k_ms_chain(ChainArgs a) {
   using C = double2;
+  __shared__ C ex[KER == 1 ? 8 * kChainThreads : 1];  // the Wilson kernel's slices (wilson_exchange)
   __shared__ MsState st;
   __shared__ __align__(16) double sp[kChainMaxParts];
   __shared__ double sh[33];
@@ -184,7 +185,11 @@ __global__ void __launch_bounds__(kChainThreads, 512 / kChainThreads) k_ms_chain
     bool first = true, stop = false;
     for (int t = blockIdx.x; t < a.np; t += gridDim.x) {
       C acc[4];
-      block_sites<double2, false, SHFL, true>(rold, a.u, g, a.am, a.imass, a.am3, t, acc);
+      const int site = t * blockDim.y + threadIdx.y;
+      if constexpr (KER == 1)
+        wilson_exchange<double2, false, false, kChainThreads, true>(rold, a.u, g, threadIdx.x, site, site < g.v3, tid,
+                                                                a.am, a.imass, a.am3, nullptr, ex, acc);
+      else block_sites<double2, false, SHFL, true>(rold, a.u, g, a.am, a.imass, a.am3, t, acc);
       if (first) {
         first = false;
         if (lam_due) {
@@ -198,7 +203,6 @@ __global__ void __launch_bounds__(kChainThreads, 512 / kChainThreads) k_ms_chain
           break;
         }
       }
-      const int site = t * blockDim.y + threadIdx.y;
       double racc = 0.0;
       if (site < g.v3) {
 #pragma unroll
@@ -217,13 +221,16 @@ __global__ void __launch_bounds__(kChainThreads, 512 / kChainThreads) k_ms_chain
     first = true;
     for (int t = blockIdx.x; t < a.np; t += gridDim.x) {
       C acc[4];
-      block_sites<double2, true, SHFL, true>(hcur, a.u, g, a.am, a.imass, a.am3, t, acc);
+      const int site = t * blockDim.y + threadIdx.y;
+      if constexpr (KER == 1)
+        wilson_exchange<double2, false, true, kChainThreads, true>(hcur, a.u, g, threadIdx.x, site, site < g.v3, tid,
+                                                                a.am, a.imass, a.am3, nullptr, ex, acc);
+      else block_sites<double2, true, SHFL, true>(hcur, a.u, g, a.am, a.imass, a.am3, t, acc);
       if (first) {
         first = false;
         ms_alpha_block(&st, rec, nstep, sum_staged(sp, a.np, tid, nthr, sh), tid);
         __syncthreads();
       }
-      const int site = t * blockDim.y + threadIdx.y;
       double racc = 0.0;
       if (site < g.v3) {
 #pragma unroll
@@ -291,7 +298,7 @@ __global__ void __launch_bounds__(kChainThreads, 512 / kChainThreads) k_ms_chain
 }
 
 // co-resident blocks of a k_ms_chain instantiation on this device (cached per device)
-template <bool SHFL>
+template <int KER, bool SHFL>
 int chain_capacity() {
   constexpr int kDevs = 64;
   static std::atomic<int> cache[kDevs];
@@ -302,15 +309,15 @@ int chain_capacity() {
     if (v > 0) return v;
   }
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ms_chain<SHFL>, kChainThreads, 0) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ms_chain<KER, SHFL>, kChainThreads, 0) != cudaSuccess) return 0;
   const int cap = occ * device_sms();
   if (dev < kDevs && cap > 0) cache[dev].store(cap, std::memory_order_relaxed);
   return cap;
 }
 
-template <bool SHFL>
+template <int KER, bool SHFL>
 int chain_launch(thr_ctx* c, const ChainArgs& a, dim3 blk, cudaStream_t st, bool dry) {
-  const int cap = chain_capacity<SHFL>();
+  const int cap = chain_capacity<KER, SHFL>();
   if (cap <= 0) return THR_ERR_UNSUPPORTED;
   // auto (mode 1): only where every site block has its own resident block; forced (2): any size
   if (c->chain_mode == 1 && a.np > cap) return THR_ERR_UNSUPPORTED;
@@ -326,7 +333,7 @@ int chain_launch(thr_ctx* c, const ChainArgs& a, dim3 blk, cudaStream_t st, bool
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_ms_chain<SHFL>, a) == cudaSuccess ? THR_OK : THR_ERR_CUDA;
+  return cudaLaunchKernelEx(&cfg, k_ms_chain<KER, SHFL>, a) == cudaSuccess ? THR_OK : THR_ERR_CUDA;
 }
 
 // THR_CHAIN_WAIT_TEST=1: every barrier expects one arrival more than the grid has, so
@@ -348,8 +355,7 @@ int ms_chain_batch(thr_ctx* c, MsState* ms, MsHist* rec, double2* ring, double2*
   const dim3 blk = stencil_block(g, kernel);
   const int nthr = (int)(blk.x * blk.y);
   const int np = (int)stencil_grid(g, kernel);
-  if (kernel != 0) return THR_ERR_UNSUPPORTED;  // the Shamir stencil only
-  // the common block shape of the stencil kernel (128 threads) with at least nt / 32 - 1
+  // the common block shape of the stencil kernels (128 threads) with at least nt / 32 - 1
   // whole warps (the sums' layout, sum_staged) and kMaxShift threads (the scalar steps)
   const int nt = kChainThreads;
   if (g.ls > nt || nthr > nt || nthr / 32 < nt / 32 - 1 || nthr < kMaxShift) return THR_ERR_UNSUPPORTED;
@@ -373,8 +379,9 @@ int ms_chain_batch(thr_ctx* c, MsState* ms, MsHist* rec, double2* ring, double2*
   a.bar = reinterpret_cast<unsigned*>(c->iscal + kIscalChainBar);
   a.extra = chain_extra();
   const bool shfl = g.ls <= 32 && (g.ls & (g.ls - 1)) == 0;
-  if (shfl) return chain_launch<true>(c, a, blk, st, dry);
-  return chain_launch<false>(c, a, blk, st, dry);
+  if (kernel == 1) return chain_launch<1, false>(c, a, blk, st, dry);
+  if (shfl) return chain_launch<0, true>(c, a, blk, st, dry);
+  return chain_launch<0, false>(c, a, blk, st, dry);
 }
 
 }  // namespace thr
