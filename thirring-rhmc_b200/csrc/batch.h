@@ -57,7 +57,7 @@ int launch_dslash_batch_fused(const BatchTable& b, int kernel, bool dag, int epi
 struct BcgRun;
 // bstep.cu: one CG step of every entry as three kernels (Shamir; entries of at most
 // kStepMaxBlocks work blocks, whose partials every block of the entry sums); step: the
-// inner solve's step, from 0.  pair_ok: FP32 storage with even Ls
+// inner solve's step, from 0
 constexpr int kStepMaxBlocks = 512;
 template <class VS, class VA>
 int launch_bcg_step(BcgRun& br, VA* r, VS* p, VS* h, VA* e, int step, int inner_cap);

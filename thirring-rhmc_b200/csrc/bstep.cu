@@ -306,6 +306,9 @@ int launch_bcg_step(BcgRun& br, VA* r, VS* p, VS* h, VA* e, int step, int inner_
   a.step = step;
   a.cap = inner_cap;
   if constexpr (sizeof(VS) == sizeof(float2)) {
+    // pairs, us per iteration with (M, M^dagger) budgets [8, 6] / 6, 5 / 5, 5 / 6, 4: 64 work blocks
+    // 17.1 16.6 16.2 16.4; 864 (eight sources on 12^3, Ls 16) 25.3 27.0 27.8 26.2; 1640 37.2 38.7
+    // 39.0 38.8; 3280 (eight on 16^3, Ls 24) 68.2 70.4 70.8 75.0; 4096 85.7 90.0 91.0 96.0
     if (t.even_ls) launch_step<VS, true, 8, 6>(a, t.total_blocks, br.st, br.pdl);
     else launch_step<VS, false, 3, 3>(a, t.total_blocks, br.st, br.pdl);
   } else {

@@ -1052,8 +1052,10 @@ int tune_lookup(const TuneKey& key, const int* cand) {
 
 // Wilson (OV false) and overlap (OV true) stencils, epilogues as launch_dslash_mode's.
 // 128-thread blocks for Ls <= 128 (register budget tuned like the Shamir kernel's), else one
-// block of up to 1024 threads per group of sites.  The exchange buffer is dynamic shared
-// memory: 8 (M) or 4 (M^dagger) values per thread.
+// block of up to 1024 threads per group of sites (64 registers; M spills 48-56 bytes).  The
+// exchange buffer is dynamic shared memory: 8 (M) or 4 (M^dagger) values per thread.  16^3, Ls
+// 130, M / M^dagger in FP64 26.2 / 21.7 us against the Q-first kernel's 32.9 / 39.1 in tuned blocks
+// of 256; Ls 160 34.1 / 27.3 (39.1 / 44.6); Ls 256 51.9 / 43.2 (57.9 / 67.7).
 template <class S, bool OV>
 int launch_wilson(const Geom& g, bool dag, S* out, const S* in, const typename Sto<S>::C* u, float am, int imass,
                   float am3, const double* zc, cudaStream_t st, const int* skip, const S* aux, const double* coef,

@@ -419,9 +419,10 @@ constexpr int kStepMaxShflBudget = 4;
 // 22.5 [18.1].  Congrad's stencils alike (343: 13.8 [12.9] 14.3 15.2 17.4; 683: 24.0 22.4 23.3
 // [19.7] 21.1).
 // Up to four blocks s -+ 1 comes by shuffles where Ls allows it (343 blocks: 8.5 against 9.4; at
-// four the M^dagger kernels with shuffles spill 20 bytes); in the registers that five or six
-// leave they spill more, and the neighbours are read (729 blocks, 18^3, Ls 16: 15.3 against
-// 16.9; 800, 20^2 x 16, Ls 16: 18.2 against 24.0).
+// four, where the M^dagger kernels with shuffles spill 20 bytes, either is within 4 %: 512
+// blocks, 16^3, Ls 16, multishift 11.9 against 11.4, congrad 15.3 against 15.8); in the registers
+// that five or six leave they spill more, and the neighbours are read (729 blocks, 18^3, Ls 16:
+// 15.3 against 16.9; 800, 20^2 x 16, Ls 16: 18.2 against 24.0).
 template <int MOST, class F>
 void with_budget(int blocks, F&& launch) {
   using std::integral_constant;
@@ -448,7 +449,10 @@ void launch_ms_step(const StepArgs<C>& a, MsState* ms, MsHist* rec, int j, cudaS
   };
   if constexpr (PER == 1) {
     with_budget<kMsStepPerSm>(a.np, go);
-  } else {  // blocks of 96 threads: six of them leave the registers a site needs
+  } else {
+    // blocks of 96 threads: six of them leave the registers a site needs.  us per iteration with
+    // budgets 2 / 4 / 6 (the rule's marked): 216 blocks [8.1] 8.1 8.6; 343 8.7 8.7 [9.3]; 549 10.1
+    // 10.1 [10.6]; 729 15.6 15.6 [10.9]; 880 17.9 18.0 [13.3]
     if (a.np <= 2 * device_sms()) go(std::integral_constant<int, 2>{});
     else go(std::integral_constant<int, 6>{});
   }
