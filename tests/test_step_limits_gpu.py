@@ -87,3 +87,26 @@ def test_batch_of_512_and_513_work_blocks():
         it_ref, _ = O.congrad(L, data[i][1], want, data[i][0], 0.3, 0.2, 1)
         assert outs[1][0][i] == it_ref and 2 < it_ref < 100
         assert rel_err(interior(outs[1][1][i]), interior(want)) <= 1e-10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(59, 10, 4, 16), (37, 8, 8, 16), (37, 12, 8, 16), (37, 16, 6, 20), (59, 10, 10, 16),
+                                  (37, 20, 8, 16)])
+def test_lead_block_in_the_wave(dims):
+    """295 and 296, 444, 592, 738 and 740 stencil blocks: with the lead block exactly two, and one
+    more than two, three, four and five per SM of 148, where the register budget steps: the
+    bits and counts of the kernel chains, multishift (FP64, FP32) and congrad."""
+    rng = np.random.default_rng(16)
+    L = O.lat(*dims)
+    u, inp = rand_links(L, rng), rand_spinor(L, rng)
+    aden, anum = np.array([1e-3, 0.05, 30.0]), np.array([0.3, 0.5, 2.0])
+    outs = []
+    with thirring.Lattice(*dims, ndiag=3) as G:
+        for stride in (0, 1 << 20):
+            G._L.thr_profile(G.h, stride, 1)
+            r = [G.multishift_solver(u, 0.05, 3, aden, anum, inp, 1e-9, 35, sp=sp) for sp in (False, True)]
+            x = np.zeros_like(inp)
+            r.append((x, G.congrad(inp, x, 1.0, 0.05, 3), 0))
+            outs.append(r)
+    for (x, it, cgr), (xc, itc, cgrc) in zip(*outs):
+        assert it == itc and np.array_equal(cgr, cgrc) and np.array_equal(x, xc)

@@ -413,7 +413,10 @@ constexpr int kStepMaxShflBudget = 4;
 
 // launch(integral_constant<int, MB>): the resident blocks per SM (2 to MOST) that a kernel's
 // registers are budgeted for: one wave of blocks with as many registers as that leaves (a
-// site's loads in flight at once).  FP64 multishift, us per iteration with budgets 2 to 6 (the
+// site's loads in flight at once).  The multishift's lead block is one of them: left over it
+// holds the next kernel up (296, 592 and 740 blocks, Ls 16: 11.7, 15.9 and 18.3 us per iteration
+// without it in the count, 8.4, 13.4 and 17.6 with); congrad's only counts the iterations (12.8,
+// 17.4 and 23.3 without, 13.4, 18.4 and 23.3 with).  FP64 multishift, us per iteration with budgets 2 to 6 (the
 // rule's marked): 343 blocks (14^3, Ls 16) 12.6 [8.5] 10.4 12.1 14.8; 549 (14^3, Ls 24) 15.9 16.4
 // [12.2] 13.3 15.5; 683 (16^3, Ls 20) 20.8 17.2 18.6 [15.2] 16.4; 820 (16^3, Ls 24) 23.5 19.5 20.3
 // 22.5 [18.1].  Congrad's stencils alike (343: 13.8 [12.9] 14.3 15.2 17.4; 683: 24.0 22.4 23.3
@@ -448,7 +451,7 @@ void launch_ms_step(const StepArgs<C>& a, MsState* ms, MsHist* rec, int j, cudaS
     launch_k(k_ms_step<C, PER, DAG, false, MB>, grd, blk, 0, st, pdl, a, ms, rec, j);
   };
   if constexpr (PER == 1) {
-    with_budget<kMsStepPerSm>(a.np, go);
+    with_budget<kMsStepPerSm>(a.np + 1, go);
   } else {
     // blocks of 96 threads: six of them leave the registers a site needs.  us per iteration with
     // budgets 2 / 4 / 6 (the rule's marked): 216 blocks [8.1] 8.1 8.6; 343 8.7 8.7 [9.3]; 549 10.1
