@@ -21,7 +21,7 @@ def _blocks(dims):
     return -(-lx * ly * lt // (128 // ls))
 
 
-def _per_sm():
+def _sms():
     import torch
     return torch.cuda.get_device_properties(0).multi_processor_count
 
@@ -44,7 +44,7 @@ def test_multishift_route_and_values(dims, sp):
     assert it == it_ref == 12
     assert rel_err(got[..., :3], want[..., :3]) <= (1e-4 if sp else 1e-10)
     chain = "%s shamir M epi=3 %dx%dx%d Ls=%d " % (("fp32" if sp else "fp64",) + dims) in _report()
-    assert chain == (_blocks(dims) + 1 > 6 * _per_sm())
+    assert chain == (_blocks(dims) + 1 > 6 * _sms())
 
 
 @pytest.mark.gpu
@@ -62,7 +62,7 @@ def test_congrad_route_and_values(dims):
         it, _ = G.congrad(phi, x, 1.0, 0.05, 3)
     assert it == it_ref and 2 < it < 100
     assert rel_err(interior(x), interior(want)) <= 1e-10
-    assert ("fp64 shamir M epi=2 %dx%dx%d Ls=%d " % dims in _report()) == (_blocks(dims) + 1 > 5 * _per_sm())
+    assert ("fp64 shamir M epi=2 %dx%dx%d Ls=%d " % dims in _report()) == (_blocks(dims) + 1 > 5 * _sms())
 
 
 @pytest.mark.gpu
